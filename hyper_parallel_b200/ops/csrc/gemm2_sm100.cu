@@ -15,19 +15,23 @@
 //   tmem_full[b] (both)     : tcgen05.commit multicast when a tile's accumulation is done
 //   tmem_empty[b] (leader)  : 8 arrivals, 4 epilogue warps of each CTA (the peer arrives remotely)
 // Operand loads are plain per-CTA TMA copies.  Every wait is bounded (see sm100_common.cuh).
+#include "epilogue_store.cuh"
 #include "gemm2_pair.cuh"
 
 namespace hpb {
 namespace g2 {
 
+constexpr int SMEM_BYTES_EPI = SMEM_BYTES + EPI_BYTES;
+
 template <bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                  const Params p) {
+                  const __grid_constant__ CUtensorMap tmap_c, const int tma_c, const Params p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+  uint8_t* epi = smem + STAGES * STAGE_BYTES;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(epi + EPI_BYTES);
   uint64_t* empty_bar = full_bar + STAGES;
   uint64_t* tmem_full = empty_bar + STAGES;   // [2]
   uint64_t* tmem_empty = tmem_full + 2;       // [2]
@@ -57,6 +61,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     fence_barrier_init();
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
+    if (!ACCUM && tma_c) tma_prefetch_desc(&tmap_c);
   }
   if (warp == 1) {
     tmem_alloc2(tmem_base_slot, TMEM_COLS);
@@ -149,8 +154,16 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   } else {
     // --------------------------------------------------------------- epilogue (both) --
     const int q = warp & 3;
-    int local_tile = 0;
+    int local_tile = 0, flip = 0;
     bool ok = true;
+    auto release = [&](int buf) {
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        if (leader) mbar_arrive(&tmem_empty[buf]);
+        else remote_arrive(mapa(smem_u32(&tmem_empty[buf]), 0));
+      }
+    };
     for (int t = cluster_id; t < num_tiles && ok; t += num_clusters, ++local_tile) {
       int m_blk, n_blk;
       tile_coords(t, num_m, num_n, m_blk, n_blk);
@@ -162,6 +175,13 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       const int row = m_blk * TILE_M + cta * CTA_M + q * 32 + lane;
       const int col0 = n_blk * TILE_N;
       const uint32_t taddr = tmem_base + buf * TILE_N + (static_cast<uint32_t>(q * 32) << 16);
+      if constexpr (!ACCUM) {
+        if (tma_c) {
+          epilogue_tma<TILE_N, OUT_F32>(&tmap_c, epi + q * EPI_WARP_BYTES, taddr, row - lane, col0, 0, p.N,
+                                        row - lane < p.M, false, lane, flip, [&] { release(buf); });
+          continue;
+        }
+      }
 #pragma unroll 1
       for (int c = 0; c < TILE_N / 32; ++c) {
         uint32_t r[32];
@@ -225,13 +245,9 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           }
         }
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) {
-        if (leader) mbar_arrive(&tmem_empty[buf]);
-        else remote_arrive(mapa(smem_u32(&tmem_empty[buf]), 0));
-      }
+      release(buf);
     }
+    if (!ACCUM && lane == 0) tma_store_wait<0>();
   }
 
   tc_fence_before();
@@ -250,17 +266,19 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p,
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || !configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES_EPI);
     if (e != cudaSuccess) return static_cast<int>(e);
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
+  CUtensorMap tc = {};
+  const int tma_c = !ACCUM && make_tmap_c(&tc, p.C, OUT_F32, p.N, p.M, 1, p.ldc) ? 1 : 0;
   const int num_tiles = ((p.M + TILE_M - 1) / TILE_M) * ((p.N + TILE_N - 1) / TILE_N);
   int clusters = num_sms / 2;
   if (num_tiles < clusters) clusters = num_tiles;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * clusters, 1, 1);
   cfg.blockDim = dim3(THREADS, 1, 1);
-  cfg.dynamicSmemBytes = SMEM_BYTES;
+  cfg.dynamicSmemBytes = SMEM_BYTES_EPI;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -269,7 +287,7 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p,
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, ta, tb, p));
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, tma_c, p));
 }
 
 

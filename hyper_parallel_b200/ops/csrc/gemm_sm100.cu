@@ -13,12 +13,14 @@
 // (one 128-byte swizzle atom of bf16), 4-stage TMA->smem ring.  Warp roles:
 //   warp 0    : TMA producer (one elected lane)
 //   warp 1    : TMEM allocator + tcgen05.mma issuer (one lane)
-//   warps 2-5 : epilogue, tcgen05.ld TMEM -> registers -> global
+//   warps 2-5 : epilogue, tcgen05.ld TMEM -> registers -> shared -> TMA store (epilogue_store.cuh);
+//               accumulating products and unaligned C take plain 16-byte loads / stores per row
 // The 512 TMEM columns hold two 128x256 fp32 accumulators, so the epilogue of
 // tile i overlaps the main loop of tile i+1.
 //
 // All waits are bounded (see sm100_common.cuh); on expiry the kernel records a
 // code in `status`, drains, frees TMEM and returns.
+#include "epilogue_store.cuh"
 #include "sm100_common.cuh"
 
 #include <mutex>
@@ -38,7 +40,7 @@ constexpr int ATOM_BYTES = 64 * BLOCK_K * 2;  // one 64-wide MN atom: 8 KB
 constexpr int GEMM_THREADS = 192;
 constexpr int TMEM_COLS = 512;
 constexpr int GROUP_M = 8;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align slack*/ + 256 /*barriers*/;
+constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_BYTES + 1024 /*align slack*/ + 256 /*barriers*/;
 
 // mode 0: plain GEMM.
 // mode 1: grouped-M.  Rows of A (and C) are grouped by expert, every group padded to a multiple
@@ -57,6 +59,7 @@ struct GemmParams {
   const int* group_offsets;
   int num_groups;
   int b_group_rows;
+  int tma_c;           // C goes out through its tensor map
 };
 
 struct TileInfo {
@@ -112,11 +115,13 @@ __device__ __forceinline__ TileInfo tile_info(int t, const GemmParams& p) {
 template <bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
-                 const __grid_constant__ CUtensorMap tmap_b, const GemmParams p) {
+                 const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_c,
+                 const GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+  uint8_t* epi = smem + STAGES * STAGE_BYTES;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(epi + EPI_BYTES);
   uint64_t* empty_bar = full_bar + STAGES;
   uint64_t* tmem_full = empty_bar + STAGES;  // [2]
   uint64_t* tmem_empty = tmem_full + 2;      // [2]
@@ -142,6 +147,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
     fence_barrier_init();
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
+    if (!ACCUM && p.tma_c) tma_prefetch_desc(&tmap_c);
   }
   if (warp == 1) {
     tmem_alloc(tmem_base_slot, TMEM_COLS);
@@ -255,7 +261,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
   } else {
     // --------------------------------------------------------- epilogue --
     const int q = warp & 3;  // TMEM lane quarter this warp may read
-    int local_tile = 0;
+    int local_tile = 0, flip = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++local_tile) {
       const TileInfo ti = tile_info(t, p);
@@ -270,6 +276,18 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
       const int col0 = ti.n0;
       const bool empty_k = ti.num_k == 0;                    // expert without tokens: the tile is zero
       const uint32_t taddr = tmem_base + buf * BLOCK_N + (static_cast<uint32_t>(q * 32) << 16);
+      if constexpr (!ACCUM) {
+        if (p.tma_c) {
+          epilogue_tma<BLOCK_N, OUT_F32>(&tmap_c, epi + q * EPI_WARP_BYTES, taddr, ti.m0 + q * 32, col0,
+                                         p.mode == 2 ? ti.group : 0, p.N, ti.m0 + q * 32 < p.M && ti.group >= 0,
+                                         empty_k, lane, flip, [&] {
+                                           tc_fence_before();
+                                           __syncwarp();
+                                           if (lane == 0) mbar_arrive(&tmem_empty[buf]);
+                                         });
+          continue;
+        }
+      }
 #pragma unroll 1
       for (int c = 0; c < BLOCK_N / 32; ++c) {
         uint32_t r[32];
@@ -342,6 +360,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
       __syncwarp();
       if (lane == 0) mbar_arrive(&tmem_empty[buf]);
     }
+    if (!ACCUM && lane == 0) tma_store_wait<0>();
   }
 
   tc_fence_before();
@@ -389,9 +408,26 @@ int make_tmap_2d(CUtensorMap* map, const void* ptr, CUtensorMapDataType dtype, i
   return r == CUDA_SUCCESS ? 0 : static_cast<int>(r);
 }
 
+bool make_tmap_c(CUtensorMap* map, void* c, bool f32, uint64_t cols, uint64_t rows, uint64_t slices, int64_t ldc) {
+  const uint64_t esize = f32 ? 4 : 2;
+  if ((reinterpret_cast<uintptr_t>(c) & 15) || (ldc * esize) % 16 || ldc < static_cast<int64_t>(cols)) return false;
+  EncodeTiledFn enc = get_encode_fn();
+  if (enc == nullptr) return false;
+  cuuint64_t dims[3] = {cols, rows, slices};
+  cuuint64_t strides[2] = {ldc * esize, ldc * esize * rows};
+  cuuint32_t box[3] = {static_cast<cuuint32_t>(128 / esize), 32, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return enc(map, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, c, dims, strides, box,
+             estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 template <bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM>
-static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int num_sms,
+static int launch(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams p, int num_sms,
                   cudaStream_t stream) {
+  CUtensorMap tc = {};
+  if (!ACCUM)
+    p.tma_c = make_tmap_c(&tc, p.C, OUT_F32, p.N, p.M, p.mode == 2 ? p.num_groups : 1, p.ldc) ? 1 : 0;
   auto kern = gemm_bf16_kernel<A_MN, B_MN, OUT_F32, ACCUM>;
   static bool configured[64] = {};
   int dev = 0;
@@ -405,7 +441,7 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams
   const int num_tiles = ((p.M + BLOCK_M - 1) / BLOCK_M) * ((p.N + BLOCK_N - 1) / BLOCK_N) *
                         (p.mode == 2 ? p.num_groups : 1);
   const int grid = num_tiles < num_sms ? num_tiles : num_sms;
-  kern<<<grid, GEMM_THREADS, SMEM_BYTES, stream>>>(ta, tb, p);
+  kern<<<grid, GEMM_THREADS, SMEM_BYTES, stream>>>(ta, tb, tc, p);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -437,7 +473,7 @@ extern "C" int hpb_gemm_bf16(const void* A, int a_mn, int64_t lda, const void* B
   else
     r = make_tmap_2d(&tb, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, N, K, ldb, 64, BLOCK_K);
   if (r) return r;
-  GemmParams p{M, N, K, C, ldc, status, 0, nullptr, nullptr, 1, 0};
+  GemmParams p{M, N, K, C, ldc, status, 0, nullptr, nullptr, 1, 0, 0};
   const int key = (a_mn ? 8 : 0) | (b_mn ? 4 : 0) | (out_f32 ? 2 : 0) | (accumulate ? 1 : 0);
   switch (key) {
 #define HPB_CASE(k, a, b, o, c) \
@@ -499,7 +535,7 @@ extern "C" int hpb_gemm_bf16_grouped(const void* A, int a_mn, int64_t lda, int64
   if (r) return r;
   // mode 2 contracts over operand rows: K carries their total count (the bound of every expert's range)
   GemmParams p{M, N, mode == 2 ? static_cast<int>(a_rows < b_rows ? a_rows : b_rows) : K, C, ldc, status, mode,
-               block_group, group_offsets, num_groups, b_group_rows};
+               block_group, group_offsets, num_groups, b_group_rows, 0};
   const int key = (a_mn ? 8 : 0) | (b_mn ? 4 : 0) | (out_f32 ? 2 : 0) | (accumulate ? 1 : 0);
   switch (key) {
 #define HPB_CASE(k, a, b, o, c) \

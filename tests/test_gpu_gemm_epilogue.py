@@ -1,0 +1,38 @@
+"""The TMA-store epilogue of the bf16 GEMMs at the edges of its 32-row x 128-byte blocks, and the
+plain-store path it leaves to unaligned outputs."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from hyper_parallel_b200.ops import functional as Fn
+from hyper_parallel_b200.ops import native
+
+# a bf16 result carries one rounding (2^-9 relative, each element); an fp32 one the order of at most
+# K additions of exact bf16 products: K * 2^-24 relative to the sum of magnitudes, below 1e-5 in 2-norm
+TOL = {torch.bfloat16: 2.0 ** -8, torch.float32: 1e-5}
+
+
+@pytest.mark.parametrize("pair", ["0", "1"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("M,N,K", [(1, 8, 8), (31, 40, 72), (33, 72, 64), (127, 264, 128), (129, 248, 200),
+                                   (257, 520, 64), (300, 1000, 24)])
+# out is a window of a larger buffer: (columns in front of it, extra columns in a row)
+@pytest.mark.parametrize("front,extra", [(0, 0), (8, 24), (1, 2), (8, 1)])
+def test_store_window(pair, dtype, M, N, K, front, extra):
+    gen = torch.Generator(device="cuda").manual_seed(M * N + K)
+    a = torch.randn(M, K, device="cuda", generator=gen).to(torch.bfloat16)
+    b = torch.randn(N, K, device="cuda", generator=gen).to(torch.bfloat16)
+    buf = torch.full((M + 2, front + N + extra), 7.0, device="cuda", dtype=dtype)
+    out = buf[1:M + 1, front:front + N]
+    Fn.set_gemm_pair_mode(pair)
+    try:
+        Fn.gemm(a, b, out=out)
+    finally:
+        Fn.set_gemm_pair_mode("auto")
+    native.check_status()
+    ref = a.double() @ b.double().t()
+    assert ((out.double() - ref).norm() / ref.norm()).item() < TOL[dtype]
+    rest = buf.clone()
+    rest[1:M + 1, front:front + N] = 7.0
+    assert (rest == 7.0).all()                 # nothing outside the window was written
