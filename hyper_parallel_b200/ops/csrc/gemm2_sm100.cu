@@ -23,10 +23,57 @@ namespace g2 {
 
 constexpr int SMEM_BYTES_EPI = SMEM_BYTES + EPI_BYTES;
 
-template <bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM>
+// Grouped (expert) products, as in gemm_sm100.cu but with 256-row blocks:
+//   mode 1: rows of A / C grouped by expert, every group padded to a multiple of 256; block_group names
+//           the expert of each block (negative: unused); B stacks b_group_rows rows per expert.
+//   mode 2: one [M, N] output per expert, the contraction over the operand rows [starts[e], ends[e]);
+//           rows from ends[e] to the next multiple of 64 behind starts[e] are zero.
+// Why pairs, although 256-row padding wastes 128 rows per expert on average where 128-row padding wastes
+// 64: the pair tile runs at 1.18 times the rate of the 128 x 256 one, so it wins from about 290 rows per
+// expert on, and mode 2 wastes nothing.
+struct Group {
+  int mode;
+  const int* block_group;
+  const int* starts;
+  const int* ends;
+  int num_groups;
+  int b_group_rows;
+};
+
+struct Tile {
+  int m_blk, n_blk, group, k_row0, num_k;
+};
+
+template <bool GROUPED>
+__device__ __forceinline__ Tile tile_at(int t, int num_m, int num_n, const Params& p, const Group& g) {
+  Tile ti;
+  if constexpr (!GROUPED) {
+    tile_coords(t, num_m, num_n, ti.m_blk, ti.n_blk);
+    ti.group = 0;
+    ti.k_row0 = 0;
+    ti.num_k = (p.K + BLOCK_K - 1) / BLOCK_K;
+  } else if (g.mode == 2) {
+    const int per = num_m * num_n;
+    ti.group = t / per;
+    tile_coords(t - ti.group * per, num_m, num_n, ti.m_blk, ti.n_blk);
+    // device-side tables: clamped to the operands' rows (p.K in this mode)
+    const int r0 = min(max(g.starts[ti.group], 0), p.K);
+    const int r1 = min(max(g.ends[ti.group], r0), p.K);
+    ti.k_row0 = r0;
+    ti.num_k = (r1 - r0 + BLOCK_K - 1) / BLOCK_K;
+  } else {
+    tile_coords(t, num_m, num_n, ti.m_blk, ti.n_blk);
+    ti.group = min(g.block_group[ti.m_blk], g.num_groups - 1);
+    ti.k_row0 = 0;
+    ti.num_k = ti.group < 0 ? 0 : (p.K + BLOCK_K - 1) / BLOCK_K;
+  }
+  return ti;
+}
+
+template <bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM, bool GROUPED>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                  const __grid_constant__ CUtensorMap tmap_c, const int tma_c, const Params p) {
+                  const __grid_constant__ CUtensorMap tmap_c, const int tma_c, const Params p, const Group g) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -43,8 +90,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   const uint32_t cta = cluster_ctarank();          // 0 = leader
   const bool leader = cta == 0;
   const int num_m = (p.M + TILE_M - 1) / TILE_M, num_n = (p.N + TILE_N - 1) / TILE_N;
-  const int num_tiles = num_m * num_n;
-  const int num_k = (p.K + BLOCK_K - 1) / BLOCK_K;
+  const int num_tiles = num_m * num_n * (GROUPED && g.mode == 2 ? g.num_groups : 1);
   const int cluster_id = blockIdx.x >> 1, num_clusters = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
@@ -80,11 +126,11 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       uint32_t phase = 0;
       bool ok = true;
       for (int t = cluster_id; t < num_tiles && ok; t += num_clusters) {
-        int m_blk, n_blk;
-        tile_coords(t, num_m, num_n, m_blk, n_blk);
-        const int m0 = m_blk * TILE_M + cta * CTA_M;       // my rows of A
-        const int n0 = n_blk * TILE_N + cta * CTA_NB;      // my rows of B
-        for (int kb = 0; kb < num_k; ++kb) {
+        const Tile ti = tile_at<GROUPED>(t, num_m, num_n, p, g);
+        const int m0 = ti.m_blk * TILE_M + cta * CTA_M;       // my rows of A
+        const int n0 = ti.n_blk * TILE_N + cta * CTA_NB;      // my rows of B
+        const int b_off = GROUPED && g.mode == 1 ? ti.group * g.b_group_rows : 0;   // the expert inside stacked B
+        for (int kb = 0; kb < ti.num_k; ++kb) {
           ok = mbar_wait_bounded(&empty_bar[stage], phase ^ 1, abort_flag, p.status, kTimeoutEmptyBarrier,
                                  blockIdx.x);
           if (!ok) break;
@@ -92,7 +138,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           uint8_t* sb = sa + A_BYTES;
           const uint32_t bar = mapa(smem_u32(&full_bar[stage]), 0);      // the leader's barrier
           if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * STAGE_BYTES);
-          const int k0 = kb * BLOCK_K;
+          const int k0 = ti.k_row0 + kb * BLOCK_K;
           if constexpr (!A_MN) {
             tma_load_2d_pair(sa, &tmap_a, bar, k0, m0);
           } else {
@@ -100,10 +146,11 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             for (int j = 0; j < CTA_M / 64; ++j) tma_load_2d_pair(sa + j * ATOM_BYTES, &tmap_a, bar, m0 + 64 * j, k0);
           }
           if constexpr (!B_MN) {
-            tma_load_2d_pair(sb, &tmap_b, bar, k0, n0);
+            tma_load_2d_pair(sb, &tmap_b, bar, k0, b_off + n0);
           } else {
 #pragma unroll
-            for (int j = 0; j < CTA_NB / 64; ++j) tma_load_2d_pair(sb + j * ATOM_BYTES, &tmap_b, bar, n0 + 64 * j, k0);
+            for (int j = 0; j < CTA_NB / 64; ++j)
+              tma_load_2d_pair(sb + j * ATOM_BYTES, &tmap_b, bar, n0 + 64 * j, b_off + k0);
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
@@ -125,6 +172,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         if (!ok) break;
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + buf * TILE_N;
+        const int num_k = tile_at<GROUPED>(t, num_m, num_n, p, g).num_k;
         for (int kb = 0; kb < num_k; ++kb) {
           ok = mbar_wait_bounded(&full_bar[stage], phase, abort_flag, p.status, kTimeoutFullBarrier, blockIdx.x);
           if (!ok) break;
@@ -165,20 +213,21 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       }
     };
     for (int t = cluster_id; t < num_tiles && ok; t += num_clusters, ++local_tile) {
-      int m_blk, n_blk;
-      tile_coords(t, num_m, num_n, m_blk, n_blk);
+      const Tile ti = tile_at<GROUPED>(t, num_m, num_n, p, g);
       const int buf = local_tile & 1;
       const uint32_t buf_phase = (local_tile >> 1) & 1;
       ok = mbar_wait_bounded(&tmem_full[buf], buf_phase, abort_flag, p.status, kTimeoutTmemFull, blockIdx.x);
       if (!ok) break;
       tc_fence_after();
-      const int row = m_blk * TILE_M + cta * CTA_M + q * 32 + lane;
-      const int col0 = n_blk * TILE_N;
+      const int row = ti.m_blk * TILE_M + cta * CTA_M + q * 32 + lane;
+      const int col0 = ti.n_blk * TILE_N;
       const uint32_t taddr = tmem_base + buf * TILE_N + (static_cast<uint32_t>(q * 32) << 16);
       if constexpr (!ACCUM) {
         if (tma_c) {
-          epilogue_tma<TILE_N, OUT_F32>(&tmap_c, epi + q * EPI_WARP_BYTES, taddr, row - lane, col0, 0, p.N,
-                                        row - lane < p.M, false, lane, flip, [&] { release(buf); });
+          epilogue_tma<TILE_N, OUT_F32>(&tmap_c, epi + q * EPI_WARP_BYTES, taddr, row - lane, col0,
+                                        GROUPED && g.mode == 2 ? ti.group : 0, p.N,
+                                        row - lane < p.M && ti.group >= 0, GROUPED && ti.num_k == 0, lane, flip,
+                                        [&] { release(buf); });
           continue;
         }
       }
@@ -259,9 +308,10 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   }
 }
 
-template <bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM>
-static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, int num_sms, cudaStream_t stream) {
-  auto kern = gemm2_bf16_kernel<A_MN, B_MN, OUT_F32, ACCUM>;
+template <bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM, bool GROUPED = false>
+static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, int num_sms, cudaStream_t stream,
+                  const Group& g = Group{}) {
+  auto kern = gemm2_bf16_kernel<A_MN, B_MN, OUT_F32, ACCUM, GROUPED>;
   static bool configured[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -271,8 +321,12 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p,
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
   CUtensorMap tc = {};
-  const int tma_c = !ACCUM && make_tmap_c(&tc, p.C, OUT_F32, p.N, p.M, 1, p.ldc) ? 1 : 0;
-  const int num_tiles = ((p.M + TILE_M - 1) / TILE_M) * ((p.N + TILE_N - 1) / TILE_N);
+  const int tma_c = !ACCUM && make_tmap_c(&tc, p.C, OUT_F32, p.N, p.M, GROUPED && g.mode == 2 ? g.num_groups : 1, p.ldc);
+  if (GROUPED && !tma_c) return -2;
+  const int64_t tiles64 = static_cast<int64_t>((p.M + TILE_M - 1) / TILE_M) * ((p.N + TILE_N - 1) / TILE_N) *
+                          (GROUPED && g.mode == 2 ? g.num_groups : 1);
+  if (tiles64 > 0x7fffffff) return -2;
+  const int num_tiles = static_cast<int>(tiles64);
   int clusters = num_sms / 2;
   if (num_tiles < clusters) clusters = num_tiles;
   cudaLaunchConfig_t cfg = {};
@@ -287,7 +341,7 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p,
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, tma_c, p));
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, tma_c, p, g));
 }
 
 
@@ -343,3 +397,34 @@ extern "C" int hpb_gemm2_bf16(const void* A, int a_mn, int64_t lda, const void* 
   return -3;
 }
 
+
+// Grouped products on CTA pairs (see Group); bf16 C, 16-byte aligned with ldc % 8 == 0.
+//   mode 1: C[M, N] = A[M, K] * B_e^T, M the padded row count; b_mn false: B [E * N, K], true: B [E * K, N].
+//   mode 2: C[e][M, N] = A[rows_e, M]^T * B[rows_e, N], both MN-major with `a_rows` rows.
+extern "C" int hpb_gemm2_bf16_grouped(const void* A, int64_t lda, int64_t a_rows, const void* B, int b_mn, int64_t ldb,
+                                      int64_t b_rows, void* C, int64_t ldc, int M, int N, int K, int mode,
+                                      const int* block_group, const int* starts, const int* ends, int num_groups,
+                                      int b_group_rows, int* status, int num_sms, cudaStream_t stream) {
+  using namespace hpb;
+  using namespace hpb::g2;
+  if (M <= 0 || N <= 0 || num_groups <= 0) return 0;
+  if (mode != 1 && mode != 2) return -4;
+  if (mode == 1 && (block_group == nullptr || M % TILE_M || K <= 0)) return -5;
+  if (mode == 2 && (starts == nullptr || ends == nullptr || !b_mn)) return -5;
+  if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15))
+    return -2;
+  cudaFree(nullptr);
+  CUtensorMap ta, tb;
+  int r;
+  if (mode == 1) r = make_tmap_2d(&ta, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, a_rows, lda, BLOCK_K, CTA_M);
+  else r = make_tmap_2d(&ta, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, M, a_rows, lda, 64, BLOCK_K);
+  if (r) return r;
+  if (!b_mn) r = make_tmap_2d(&tb, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, b_rows, ldb, BLOCK_K, CTA_NB);
+  else r = make_tmap_2d(&tb, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, N, b_rows, ldb, 64, BLOCK_K);
+  if (r) return r;
+  Params p{M, N, mode == 2 ? static_cast<int>(a_rows < b_rows ? a_rows : b_rows) : K, C, ldc, status};
+  const Group g{mode, block_group, starts, ends, num_groups, b_group_rows};
+  if (mode == 2) return g2::launch<true, true, false, false, true>(ta, tb, p, num_sms, stream, g);
+  if (b_mn) return g2::launch<false, true, false, false, true>(ta, tb, p, num_sms, stream, g);
+  return g2::launch<false, false, false, false, true>(ta, tb, p, num_sms, stream, g);
+}

@@ -177,6 +177,10 @@ def expert_parallel_ffn(x: torch.Tensor, topk_idx: torch.Tensor, topk_w: torch.T
     H = x.shape[-1]
     ep = cc.group_size(ep_group)
     e_local = num_experts // ep
+    if ep == 1 and native.use_native(x):
+        from . import grouped
+        if grouped.local_experts_usable(x, topk_idx, topk_w, w_gate_up, w_down, num_experts):
+            return grouped.local_experts(x, topk_idx, topk_w, w_gate_up, w_down)
     flat_e = topk_idx.reshape(-1)
     order = torch.argsort(flat_e, stable=True)                 # pair ids sorted by expert
     token_of = order // k
