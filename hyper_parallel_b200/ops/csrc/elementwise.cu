@@ -1,6 +1,6 @@
 // Memory-bound kernels of the transformer step (sm_100a): RMSNorm fwd/bwd (with
-// optional fused residual add), SwiGLU fwd/bwd, RoPE fwd/bwd, fused softmax
-// cross-entropy fwd+bwd, and the fused AdamW update with fp32 master weights.
+// optional fused residual add), SwiGLU fwd/bwd, RoPE fwd/bwd, and the fused AdamW
+// update with fp32 master weights.
 // All of them stream their operands exactly once with 16-byte accesses; the
 // roofline for each is bytes / HBM bandwidth.
 #include <cuda_bf16.h>
@@ -18,11 +18,6 @@ __device__ __forceinline__ float warp_sum(float v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
 // Block-wide sum; `red` is >= 32 floats of shared memory.  All threads get the result.
 __device__ __forceinline__ float block_sum(float v, float* red) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
@@ -32,15 +27,6 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
   __syncthreads();
   float t = (lane < nw) ? red[lane] : 0.f;
   return warp_sum(t);
-}
-__device__ __forceinline__ float block_max(float v, float* red) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-  v = warp_max(v);
-  __syncthreads();
-  if (lane == 0) red[warp] = v;
-  __syncthreads();
-  float t = (lane < nw) ? red[lane] : -INFINITY;
-  return warp_max(t);
 }
 __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
   const bf162* p = reinterpret_cast<const bf162*>(&u);
@@ -351,61 +337,6 @@ __global__ void rope_vec_kernel(bf16* __restrict__ x, const float2* __restrict__
   }
 }
 
-// ------------------------------------------------------- cross entropy ----
-// One CTA per token row.  Reads logits[row, :V] (bf16), writes loss[row] (fp32) and
-// overwrites the row IN PLACE with d(loss_sum * grad_scale)/dlogits =
-// (softmax - onehot) * grad_scale.  Rows with target < 0 get zero loss and gradient.
-constexpr int CE_THREADS = 1024;
-__global__ void __launch_bounds__(CE_THREADS)
-cross_entropy_fwd_bwd_kernel(bf16* __restrict__ logits, const int64_t* __restrict__ target,
-                             float* __restrict__ loss, int V, int64_t ld, float grad_scale) {
-  __shared__ float red[32];
-  const int64_t row = blockIdx.x;
-  bf16* lr = logits + row * ld;
-  const int64_t tgt = target[row];
-  const int nvec = V >> 3;
-  uint4* lv = reinterpret_cast<uint4*>(lr);
-  float mx = -INFINITY;
-  for (int c = threadIdx.x; c < nvec; c += CE_THREADS) {
-    float f[8];
-    unpack8(lv[c], f);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) mx = fmaxf(mx, f[e]);
-  }
-  for (int c = nvec * 8 + threadIdx.x; c < V; c += CE_THREADS) mx = fmaxf(mx, __bfloat162float(lr[c]));
-  mx = block_max(mx, red);
-  float se = 0.f;
-  for (int c = threadIdx.x; c < nvec; c += CE_THREADS) {
-    float f[8];
-    unpack8(lv[c], f);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) se += __expf(f[e] - mx);
-  }
-  for (int c = nvec * 8 + threadIdx.x; c < V; c += CE_THREADS) se += __expf(__bfloat162float(lr[c]) - mx);
-  se = block_sum(se, red);
-  const float lse = mx + __logf(se);
-  const bool valid = tgt >= 0 && tgt < V;
-  if (threadIdx.x == 0) loss[row] = valid ? lse - __bfloat162float(lr[tgt]) : 0.f;
-  __syncthreads();
-  const float gs = valid ? grad_scale : 0.f;
-  for (int c = threadIdx.x; c < nvec; c += CE_THREADS) {
-    float f[8];
-    unpack8(lv[c], f);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      float pr = __expf(f[e] - lse);
-      if (c * 8 + e == tgt) pr -= 1.f;
-      f[e] = pr * gs;
-    }
-    lv[c] = pack8(f);
-  }
-  for (int c = nvec * 8 + threadIdx.x; c < V; c += CE_THREADS) {
-    float pr = __expf(__bfloat162float(lr[c]) - lse);
-    if (c == tgt) pr -= 1.f;
-    lr[c] = __float2bfloat16(pr * gs);
-  }
-}
-
 // ---------------------------------------------------------------- AdamW ----
 // Flat fused update with fp32 master weights (decoupled weight decay):
 //   g = grad * grad_scale ; m = b1 m + (1-b1) g ; v = b2 v + (1-b2) g^2
@@ -558,15 +489,6 @@ extern "C" int hpb_rope(void* x, const int* pos, int64_t T, int S, int NH, int D
   if (T == 0) return 0;
   rope_kernel<<<grid_for(T * NH * (D / 2), 256, num_sms), 256, 0, s>>>(
       (bf16*)x, pos, T, S, NH, D, ld, log2f(theta), backward ? -1.f : 1.f);
-  return static_cast<int>(cudaGetLastError());
-}
-
-extern "C" int hpb_cross_entropy(void* logits, const int64_t* target, float* loss, int64_t T, int V,
-                                 int64_t ld, float grad_scale, cudaStream_t s) {
-  if (ld % 8 || (reinterpret_cast<uintptr_t>(logits) & 15)) return -2;
-  if (T == 0) return 0;
-  cross_entropy_fwd_bwd_kernel<<<static_cast<unsigned>(T), CE_THREADS, 0, s>>>(
-      (bf16*)logits, target, loss, V, ld, grad_scale);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -464,7 +464,8 @@ def cross_entropy_fwd_bwd(logits: torch.Tensor, target: torch.Tensor,
     loss = torch.empty(T, dtype=torch.float32, device=logits.device)
     rc = native.lib().hpb_cross_entropy(logits.data_ptr(), target.data_ptr(), loss.data_ptr(), T, V,
                                         logits.stride(0), float(grad_scale),
-                                        native.stream(logits.device))
+                                        native.status_word(logits.device).data_ptr(),
+                                        native.sm_count(logits.device), native.stream(logits.device))
     native.check(rc, "hpb_cross_entropy")
     return loss
 
