@@ -248,7 +248,8 @@ class _RMSNorm(torch.autograd.Function):
         dy2 = dy.reshape(T, H).contiguous()
         dh2 = dh.reshape(T, H).contiguous() if (ctx.has_res and dh is not None) else None
         dx = torch.empty_like(src)
-        P = min(T, native.sm_count(src.device) * 8)
+        # partial rows of dw = CTAs: about 1024 threads per SM (a CTA has as many as hold a row)
+        P = min(T, native.sm_count(src.device) * (8 if H <= 1024 else 4 if H <= 2048 else 2))
         part = torch.empty((P, H), dtype=torch.float32, device=src.device)
         dw = torch.empty_like(w)
         rc = native.lib().hpb_rmsnorm_bwd(dy2.data_ptr(), src.data_ptr(), w.data_ptr(), rstd.data_ptr(),
