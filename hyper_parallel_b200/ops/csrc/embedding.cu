@@ -6,12 +6,16 @@
 // memory).  No sort over the tokens and no floating-point atomics:
 //
 //   1. count   cnt[v] += 1 per token (integer atomics: the result does not depend on the order)
-//   2. scan    off[v] = exclusive prefix sum of cnt over the vocabulary (one CTA)
+//   2. scan    off[v] = exclusive prefix sum of cnt over the vocabulary: sums of 1024 counts, then every
+//              CTA adds up the sums in front of its 1024 and scans them (one CTA that walked the whole
+//              vocabulary took 280 us for 128256 rows; the two launches take 7)
 //   3. fill    bucket[off[v] + k] = t, k handed out by an integer atomic (order inside a bucket varies)
-//   4. sum     one CTA per vocabulary row: the bucket is rank-sorted by token index in shared memory
-//              (token indices are distinct, buckets are short), then the rows are added in that
-//              order -- the same order, hence the same bits, on every run.  Buckets longer than
-//              kMaxSorted tokens are added in bucket order (still correct, order not fixed).
+//   4. sum     one CTA per vocabulary row and 256 of its vectors: the bucket is rank-sorted by token index
+//              in shared memory (token indices are distinct, buckets are short), then the rows are added in
+//              that order -- the same order, hence the same bits, on every run.  Buckets longer than
+//              kMaxSorted tokens are added in bucket order (still correct, order not fixed).  Bound by
+//              writing dW (238 us for 128256 x 4096 and 8192 Zipf-distributed tokens, 370 us before); a CTA fetches the counts of kSumRows rows at once, so that the many rows without a
+//              token cost no load latency each, and keeps eight rows of a long bucket in flight.
 //
 // Indices outside [0, V) contribute nothing (forward: a zero row) and record kBadArgument in the
 // status word.
@@ -51,86 +55,125 @@ __global__ void embed_count_kernel(const int64_t* __restrict__ idx, int* __restr
   }
 }
 
-// off[v] = sum of cnt[0..v); cursor[v] = 0.  One CTA of 1024 threads, each scanning a contiguous chunk.
-__global__ void __launch_bounds__(1024) embed_scan_kernel(const int* __restrict__ cnt, int* __restrict__ off,
-                                                          int* __restrict__ cursor, int V) {
-  __shared__ int part[1024];
-  const int chunk = (V + 1023) / 1024;
-  const int lo = min(static_cast<int>(threadIdx.x) * chunk, V), hi = min(lo + chunk, V);
-  int s = 0;
-  for (int v = lo; v < hi; ++v) s += cnt[v];
-  part[threadIdx.x] = s;
+constexpr int kScan = 1024;      // counts per CTA of the scan
+constexpr int kSumRows = 8;      // vocabulary rows per CTA of the sum
+
+__device__ __forceinline__ int block_sum_1024(int v, int* red) {      // every thread gets the sum
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
-  // inclusive Hillis-Steele scan of the 1024 partial sums
-  for (int d = 1; d < 1024; d <<= 1) {
-    const int add = threadIdx.x >= d ? part[threadIdx.x - d] : 0;
-    __syncthreads();
-    part[threadIdx.x] += add;
-    __syncthreads();
-  }
-  int run = part[threadIdx.x] - s;
-  for (int v = lo; v < hi; ++v) {
-    off[v] = run;
-    run += cnt[v];
-    cursor[v] = 0;
-  }
+  v = red[threadIdx.x & 31];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  __syncthreads();
+  return v;
 }
 
-__global__ void embed_fill_kernel(const int64_t* __restrict__ idx, const int* __restrict__ off, int* __restrict__ cursor,
-                                  int* __restrict__ bucket, int64_t T, int V) {
+// part[b] = sum of the 1024 counts of block b
+__global__ void __launch_bounds__(kScan) embed_part_kernel(const int* __restrict__ cnt, int* __restrict__ part, int V) {
+  __shared__ int red[32];
+  const int v = blockIdx.x * kScan + threadIdx.x;
+  const int s = block_sum_1024(v < V ? cnt[v] : 0, red);
+  if (threadIdx.x == 0) part[blockIdx.x] = s;
+}
+
+// off[v] = cursor[v] = sum of cnt[0..v)
+__global__ void __launch_bounds__(kScan) embed_scan_kernel(const int* __restrict__ cnt, const int* __restrict__ part,
+                                                           int* __restrict__ off, int* __restrict__ cursor, int V) {
+  __shared__ int red[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int before = 0;
+  for (int b = threadIdx.x; b < static_cast<int>(blockIdx.x); b += kScan) before += part[b];
+  before = block_sum_1024(before, red);
+  const int v = blockIdx.x * kScan + threadIdx.x;
+  const int n = v < V ? cnt[v] : 0;
+  int inc = n;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int up = __shfl_up_sync(0xffffffffu, inc, d);
+    if (lane >= d) inc += up;
+  }
+  if (lane == 31) red[warp] = inc;
+  __syncthreads();
+  int w = lane < warp ? red[lane] : 0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+  if (v < V) off[v] = cursor[v] = before + w + inc - n;
+}
+
+__global__ void embed_fill_kernel(const int64_t* __restrict__ idx, int* __restrict__ cursor, int* __restrict__ bucket,
+                                  int64_t T, int V) {
   for (int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < T;
        t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int64_t v = idx[t];
     if (v < 0 || v >= V) continue;
-    bucket[off[v] + atomicAdd(&cursor[v], 1)] = static_cast<int>(t);
+    bucket[atomicAdd(&cursor[v], 1)] = static_cast<int>(t);
   }
 }
 
-// One CTA per vocabulary row (grid-stride); thread c owns the 16-byte vector c, c + blockDim.x, ... of the row.
+__device__ __forceinline__ void add_row(float (&acc)[8], const uint4& x) {
+  const __nv_bfloat162* xb = reinterpret_cast<const __nv_bfloat162*>(&x);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float2 f = __bfloat1622float2(xb[e]);
+    acc[2 * e] += f.x;
+    acc[2 * e + 1] += f.y;
+  }
+}
+
+// kSumRows vocabulary rows per CTA, a `stride` apart: ids follow frequency in most vocabularies, so that
+// neighbouring rows have long buckets together (eight consecutive rows: 566 us for 8192 Zipf-distributed
+// tokens, the first CTAs being the tail).  Thread c owns the 16-byte vector blockIdx.y * 256 + c.
 __global__ void __launch_bounds__(256) embed_sum_kernel(const uint4* __restrict__ dy, const int* __restrict__ cnt,
                                                         const int* __restrict__ off, const int* __restrict__ bucket,
-                                                        uint4* __restrict__ dw, int V, int vec_per_row) {
+                                                        uint4* __restrict__ dw, int V, int stride, int vec_per_row) {
   __shared__ int raw[kMaxSorted];
   __shared__ int sorted[kMaxSorted];
-  for (int v = blockIdx.x; v < V; v += gridDim.x) {
-    const int n = cnt[v];
-    uint4* dst = dw + static_cast<int64_t>(v) * vec_per_row;
-    if (n == 0) {
-      for (int c = threadIdx.x; c < vec_per_row; c += blockDim.x) dst[c] = make_uint4(0, 0, 0, 0);
-      continue;
-    }
-    const int* b = bucket + off[v];
-    const int* order = b;
-    if (n <= kMaxSorted) {
-      __syncthreads();                       // the previous row's readers are done with the arrays
-      for (int i = threadIdx.x; i < n; i += blockDim.x) raw[i] = b[i];
-      __syncthreads();
-      for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const int t = raw[i];
-        int rank = 0;
-        for (int j = 0; j < n; ++j) rank += raw[j] < t;
-        sorted[rank] = t;
-      }
-      __syncthreads();
-      order = sorted;
-    }
-    for (int c = threadIdx.x; c < vec_per_row; c += blockDim.x) {
-      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      for (int i = 0; i < n; ++i) {
-        const uint4 x = dy[static_cast<int64_t>(order[i]) * vec_per_row + c];
-        const __nv_bfloat162* xb = reinterpret_cast<const __nv_bfloat162*>(&x);
+  const int c = blockIdx.y * 256 + threadIdx.x;
+  const bool live = c < vec_per_row;
+  for (int v0 = blockIdx.x; v0 < stride; v0 += gridDim.x) {
+    int counts[kSumRows];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 f = __bfloat1622float2(xb[e]);
-          acc[2 * e] += f.x;
-          acc[2 * e + 1] += f.y;
+    for (int i = 0; i < kSumRows; ++i) counts[i] = v0 + i * static_cast<int64_t>(stride) < V ? cnt[v0 + i * stride] : -1;
+#pragma unroll
+    for (int i = 0; i < kSumRows; ++i)
+      if (counts[i] == 0 && live) dw[static_cast<int64_t>(v0 + i * stride) * vec_per_row + c] = make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int i = 0; i < kSumRows; ++i) {
+      const int n = counts[i];
+      if (n <= 0) continue;                    // uniform over the CTA
+      const int* b = bucket + off[v0 + i * stride];
+      const int* order = b;
+      if (n > 1 && n <= kMaxSorted) {
+        __syncthreads();                       // the previous row's readers are done with the arrays
+        for (int k = threadIdx.x; k < n; k += 256) raw[k] = b[k];
+        __syncthreads();
+        for (int k = threadIdx.x; k < n; k += 256) {
+          const int t = raw[k];
+          int rank = 0;
+          for (int j = 0; j < n; ++j) rank += raw[j] < t;
+          sorted[rank] = t;
         }
+        __syncthreads();
+        order = sorted;
       }
+      if (!live) continue;
+      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      int k = 0;
+      for (; k + 8 <= n; k += 8) {
+        uint4 x[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) x[u] = dy[static_cast<int64_t>(order[k + u]) * vec_per_row + c];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) add_row(acc, x[u]);
+      }
+      for (; k < n; ++k) add_row(acc, dy[static_cast<int64_t>(order[k]) * vec_per_row + c]);
       uint4 o;
       __nv_bfloat162* ob = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
       for (int e = 0; e < 4; ++e) ob[e] = __floats2bfloat162_rn(acc[2 * e], acc[2 * e + 1]);
-      dst[c] = o;
+      dw[static_cast<int64_t>(v0 + i * stride) * vec_per_row + c] = o;
     }
   }
 }
@@ -155,7 +198,9 @@ extern "C" int hpb_embedding_fwd(const int64_t* idx, const void* w, void* out, i
 }
 
 // Number of int32 words of scratch that hpb_embedding_bwd needs.
-extern "C" int64_t hpb_embedding_bwd_scratch_words(int64_t T, int V) { return 3ll * V + T; }
+extern "C" int64_t hpb_embedding_bwd_scratch_words(int64_t T, int V) {
+  return 3ll * V + T + (V + hpb::emb::kScan - 1) / hpb::emb::kScan;
+}
 
 // dw[V, H] = scatter-add of dy[T, H] by idx (every row written); scratch: hpb_embedding_bwd_scratch_words ints.
 extern "C" int hpb_embedding_bwd(const int64_t* idx, const void* dy, void* dw, int* scratch, int64_t T, int V, int H,
@@ -166,6 +211,8 @@ extern "C" int hpb_embedding_bwd(const int64_t* idx, const void* dy, void* dw, i
   int* off = scratch + V;
   int* cursor = scratch + 2ll * V;
   int* bucket = scratch + 3ll * V;
+  int* part = bucket + T;
+  const int scan_blocks = (V + emb::kScan - 1) / emb::kScan;
   cudaError_t e = cudaMemsetAsync(cnt, 0, sizeof(int) * static_cast<size_t>(V), s);
   if (e != cudaSuccess) return static_cast<int>(e);
   const int sms = num_sms > 0 ? num_sms : 148;
@@ -174,14 +221,16 @@ extern "C" int hpb_embedding_bwd(const int64_t* idx, const void* dy, void* dw, i
     emb::embed_count_kernel<<<static_cast<unsigned>(want < sms * 8 ? want : sms * 8), 256, 0, s>>>(idx, cnt, T, V,
                                                                                                  status);
   }
-  emb::embed_scan_kernel<<<1, 1024, 0, s>>>(cnt, off, cursor, V);
+  emb::embed_part_kernel<<<scan_blocks, emb::kScan, 0, s>>>(cnt, part, V);
+  emb::embed_scan_kernel<<<scan_blocks, emb::kScan, 0, s>>>(cnt, part, off, cursor, V);
   if (T > 0) {
     const int64_t want = (T + 255) / 256;
-    emb::embed_fill_kernel<<<static_cast<unsigned>(want < sms * 8 ? want : sms * 8), 256, 0, s>>>(idx, off, cursor,
-                                                                                                bucket, T, V);
+    emb::embed_fill_kernel<<<static_cast<unsigned>(want < sms * 8 ? want : sms * 8), 256, 0, s>>>(idx, cursor, bucket,
+                                                                                                T, V);
   }
-  const int rows = V < sms * 32 ? V : sms * 32;
-  emb::embed_sum_kernel<<<rows, 256, 0, s>>>(reinterpret_cast<const uint4*>(dy), cnt, off, bucket,
-                                             reinterpret_cast<uint4*>(dw), V, H / 8);
+  const int groups = (V + emb::kSumRows - 1) / emb::kSumRows;
+  const dim3 grid(groups < sms * 32 ? groups : sms * 32, (H / 8 + 255) / 256);
+  emb::embed_sum_kernel<<<grid, 256, 0, s>>>(reinterpret_cast<const uint4*>(dy), cnt, off, bucket,
+                                             reinterpret_cast<uint4*>(dw), V, groups, H / 8);
   return static_cast<int>(cudaGetLastError());
 }

@@ -427,7 +427,7 @@ class _Embedding(torch.autograd.Function):
         dev = dy2.device
         T = idx.numel()
         dw = torch.empty((V, H), dtype=dy2.dtype, device=dev)
-        scratch = torch.empty(3 * V + T, dtype=torch.int32, device=dev)
+        scratch = torch.empty(3 * V + T + (V + 1023) // 1024, dtype=torch.int32, device=dev)
         rc = native.lib().hpb_embedding_bwd(idx.data_ptr(), dy2.data_ptr(), dw.data_ptr(), scratch.data_ptr(), T, V, H,
                                             native.status_word(dev).data_ptr(), native.sm_count(dev), native.stream(dev))
         native.check(rc, "hpb_embedding_bwd")
