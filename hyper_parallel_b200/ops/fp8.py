@@ -38,6 +38,12 @@ def _lib():
     return lib
 
 
+def _vectors(t: torch.Tensor) -> torch.Tensor:
+    """``t`` contiguous on a 16-byte boundary: the quantisers read 16-byte vectors."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def quantize_act_1x128(x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
     """``x[M, K]`` bf16 -> (e4m3 ``[M, K]``, scales ``[K/128, M]`` fp32)."""
     M, K = x.shape
@@ -47,7 +53,7 @@ def quantize_act_1x128(x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
         scale = xb.abs().amax(-1).clamp_min(1e-10) / E4M3_MAX
         q = (xb / scale[..., None]).to(torch.float8_e4m3fn).view(M, K)
         return q, scale.t().contiguous()
-    x = x.contiguous()
+    x = _vectors(x)
     q = torch.empty((M, K), dtype=torch.float8_e4m3fn, device=x.device)
     s = torch.empty((K // 128, M), dtype=torch.float32, device=x.device)
     native.check(_lib().hpb_quant_act_1x128(x.data_ptr(), q.data_ptr(), s.data_ptr(), M, K, native.stream(x.device)),
@@ -66,7 +72,7 @@ def quantize_weight_128x128(w: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor
         scale = wp.abs().amax(dim=(1, 3)).clamp_min(1e-10) / E4M3_MAX
         q = (wp / scale[:, None, :, None]).to(torch.float8_e4m3fn).view(nb * 128, K)[:N]
         return q.contiguous(), scale
-    w = w.contiguous()
+    w = _vectors(w)
     q = torch.empty((N, K), dtype=torch.float8_e4m3fn, device=w.device)
     s = torch.empty((nb, K // 128), dtype=torch.float32, device=w.device)
     native.check(_lib().hpb_quant_weight_128x128(w.data_ptr(), q.data_ptr(), s.data_ptr(), N, K,
