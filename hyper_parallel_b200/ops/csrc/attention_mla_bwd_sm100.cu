@@ -114,7 +114,7 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(drain_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform(threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   // (batch, head) pairs are processed in groups of `head_group`: the CTAs that run at the same time
   // then add into a few MB of the fp32 dQ (and re-read the same Q / dO), which stays in L2; inside
@@ -174,7 +174,7 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_base_slot;
+  const uint32_t tmem_base = uniform(*tmem_base_slot);
   // tensor-memory columns
   constexpr uint32_t COL_ST = 0;      // 64
   constexpr uint32_t COL_DPT = 64;    // 64
@@ -231,13 +231,14 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------- MMA issuer --
-    if (lane == 0 && n_it > 0) {
+    if (n_it > 0) {      // the whole warp walks the loop, one elected lane issues
+      const bool issuer = elect_one();
       constexpr uint32_t idesc_st = make_idesc(1, 1, 0, 0, BN, BQ);    // K / V (K-major) x Q / dO (K-major)
       constexpr uint32_t idesc_dv = make_idesc(1, 1, 0, 1, BN, DV);    // P^T (K-major) x dO (MN-major)
       constexpr uint32_t idesc_dk = make_idesc(1, 1, 0, 1, BN, DQK);   // dS^T (K-major) x Q (MN-major)
       constexpr uint32_t idesc_dq = make_idesc(1, 1, 1, 1, 128, BQ);   // K^T (MN-major) x dS^T (MN-major)
-      const uint32_t k_addr = smem_u32(sK), v_addr = smem_u32(sV), q_addr = smem_u32(sQ), do_addr = smem_u32(sDO),
-                     ds_addr = smem_u32(sDS);
+      const uint32_t k_addr = uniform(smem_u32(sK)), v_addr = uniform(smem_u32(sV)), q_addr = uniform(smem_u32(sQ)),
+                     do_addr = uniform(smem_u32(sDO)), ds_addr = uniform(smem_u32(sDS));
       bool ok = true;
       const uint64_t k_desc = make_smem_desc_sw128(k_addr, 0, 1024);               // K as K-major A
       const uint64_t v_desc = make_smem_desc_sw128(v_addr, 0, 1024);               // V as K-major A
@@ -249,12 +250,13 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       const uint64_t dsk_desc = make_smem_desc_sw128(ds_addr, 0, 1024);            // dS^T as K-major A
       const uint64_t dsm_desc = make_smem_desc_sw128(ds_addr, PT_BYTES, 1024);     // dS^T as MN-major B
       auto wait_on = [&](uint64_t* bar, uint32_t parity, int code) {
-        return mbar_wait_bounded(bar, parity, abort_flag, p.status, code, blockIdx.x);
+        return mbar_wait_warp(bar, parity, abort_flag, p.status, code, blockIdx.x);
       };
       auto q_ready = [&](int it) { return wait_on(&q_full[it % RING], (it / RING) & 1, kTimeoutFullBarrier); };
       auto do_ready = [&](int it) { return wait_on(&do_full[it % RING], (it / RING) & 1, kTimeoutFullBarrier); };
       // S^T(it) = K Q^T: 3 units of 64 columns, 4 steps of 16 columns (32 bytes) each
       auto issue_st = [&](int it) {
+        if (!issuer) return;
         const uint64_t qa = desc_at(qk_desc, (it % RING) * Q_BYTES);
         if (!(p.probe & 16))
 #pragma unroll
@@ -267,6 +269,7 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       };
       // dP^T(it) = V dO^T
       auto issue_dpt = [&](int it) {
+        if (!issuer) return;
         const uint64_t doa = desc_at(dok_desc, (it % RING) * DO_BYTES);
         if (!(p.probe & 16))
 #pragma unroll
@@ -296,7 +299,7 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
           issue_st(1);
         }
       }
-      const bool prof = p.prof != nullptr && blockIdx.x == 0;
+      const bool prof = p.prof != nullptr && blockIdx.x == 0 && issuer;
       long long acc[5] = {0, 0, 0, 0, 0};
       long long tp = prof ? clock64() : 0;
       auto tick = [&](int i) {
@@ -319,12 +322,12 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         const uint32_t first = it ? 1u : 0u;
         // dV += P^T dO (contraction over the 64 query rows: 4 steps of 16).  P^T lies in the dP^T
         // buffer: query rows 0..31 in columns 0..15, 32..63 in columns 32..47 (8 columns per step)
-        if (!(p.probe & 8))
+        if (issuer && !(p.probe & 8))
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
           umma_f16_ts(tmem_base + COL_DV, tmem_base + COL_DPT + (kk >> 1) * 32 + (kk & 1) * 8, desc_at(doa, kk * 2048),
                       idesc_dv, kk ? 1u : first);
-        umma_commit(&do_empty[it % RING]);
+        if (issuer) umma_commit(&do_empty[it % RING]);
         // dP^T of the next step: its softmax is waiting for nothing else (executes behind dV, which
         // reads the buffer it overwrites)
         if (it + 1 < n_it) {
@@ -334,11 +337,11 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
           issue_dpt(it + 1);
         }
         // dK += dS^T Q; frees the Q slot, so that the load of step it + 2 starts early
-        if (!(p.probe & 8))
+        if (issuer && !(p.probe & 8))
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
           umma_f16(tmem_base + COL_DK, desc_at(dsa, kk * 32), desc_at(qa, kk * 2048), idesc_dk, kk ? 1u : first);
-        umma_commit(&q_empty[it % RING]);
+        if (issuer) umma_commit(&q_empty[it % RING]);
         tick(1);
         // dQ^T = K^T dS^T (contraction over the 128 key rows: 8 steps of 16).  Head elements 64..191
         // (units 1, 2 of K) go into the S^T buffer, free once the scores of step it + 1 are in
@@ -349,12 +352,12 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
           tc_fence_after();
         }
         tick(2);
-        if (!(p.probe & 4))
+        if (issuer && !(p.probe & 4))
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)
           umma_f16(tmem_base + COL_ST, desc_at(kt_desc, UNIT_BYTES + kk * 2048), desc_at(dsm, kk * 2048), idesc_dq,
                    kk ? 1u : 0u);
-        umma_commit(dq_hi_full);
+        if (issuer) umma_commit(dq_hi_full);
         // head elements 0..127 (units 0, 1 of K) go into the dQ^T buffer, free once the tile of the
         // step before was read; this product runs while the upper tile is read out
         if (it > 0) {
@@ -362,12 +365,12 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
           if (!ok) break;
           tc_fence_after();
         }
-        if (!(p.probe & 4))
+        if (issuer && !(p.probe & 4))
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)
           umma_f16(tmem_base + COL_DQ, desc_at(kt_desc, kk * 2048), desc_at(dsm, kk * 2048), idesc_dq, kk ? 1u : 0u);
-        umma_commit(dq_lo_full);
-        umma_commit(&pt_free[b]);     // every reader of dS^T of this step has been issued
+        if (issuer) umma_commit(dq_lo_full);
+        if (issuer) umma_commit(&pt_free[b]);     // every reader of dS^T of this step has been issued
         tick(3);
         // The upper tile must have left the S^T buffer before anything else is written there: S^T of
         // step it + 2, or -- in the last two steps, where no score tile follows -- the upper tile of
@@ -386,8 +389,8 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       }
       if (prof)
         for (int i = 0; i < 5; ++i) p.prof[10 + i] = acc[i];
-      if (ok) umma_commit(acc_full);
-      if (!ok) {
+      if (ok && issuer) umma_commit(acc_full);
+      if (!ok && issuer) {
         umma_commit(drain_bar);
         const uint64_t t0 = globaltimer_ns();
         while (!mbar_try_wait(drain_bar, 0) && globaltimer_ns() - t0 < 100000000ull) {}

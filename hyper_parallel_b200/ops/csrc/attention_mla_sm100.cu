@@ -81,7 +81,7 @@ mla_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(drain_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform(threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
 
   // heavy (late) query blocks first: they have the most key tiles under a causal mask
@@ -120,7 +120,7 @@ mla_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_base_slot;
+  const uint32_t tmem_base = uniform(*tmem_base_slot);
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer --
@@ -166,26 +166,29 @@ mla_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------- MMA issuer --
-    if (lane == 0 && n_kv > 0) {
+    if (n_kv > 0) {      // the whole warp walks the loop, one elected lane issues
+      const bool issuer = elect_one();
       constexpr uint32_t idesc_s = make_idesc(1, 1, 0, 0, BM, BN);   // Q (K-major) x K (K-major)
       constexpr uint32_t idesc_o = make_idesc(1, 1, 0, 1, BM, DV);   // P (tensor memory) x V (MN-major)
       const int nt[2] = {n0, n1};
       bool ok = true;
-      const uint64_t q_desc = make_smem_desc_sw128(smem_u32(sQ), 0, 1024);
-      const uint64_t k_desc = make_smem_desc_sw128(smem_u32(sRing), 0, 1024);                  // K unit, K-major
-      const uint64_t v_desc = make_smem_desc_sw128(smem_u32(sRing), UNIT_BYTES / 2, 1024);     // V unit, MN-major
+      const uint64_t q_desc = make_smem_desc_sw128(uniform(smem_u32(sQ)), 0, 1024);
+      const uint64_t k_desc = make_smem_desc_sw128(uniform(smem_u32(sRing)), 0, 1024);                  // K unit, K-major
+      const uint64_t v_desc = make_smem_desc_sw128(uniform(smem_u32(sRing)), UNIT_BYTES / 2, 1024);     // V unit, MN-major
       auto wait_units = [&](int first, int count) {
         bool good = true;
         for (int u = first; u < first + count && good; ++u)
-          good = mbar_wait_bounded(&u_full[u % RING], (u / RING) & 1, abort_flag, p.status, kTimeoutFullBarrier,
+          good = mbar_wait_warp(&u_full[u % RING], (u / RING) & 1, abort_flag, p.status, kTimeoutFullBarrier,
                                    blockIdx.x);
         return good;
       };
       auto free_units = [&](int first, int count) {
+        if (!issuer) return;
         for (int u = first; u < first + count; ++u) umma_commit(&u_empty[u % RING]);
       };
       // S_t = Q_t K_j^T: 3 units of 64 columns, 4 steps of 16 columns (32 bytes) each
       auto issue_s = [&](int t, int j) {
+        if (!issuer) return;
         const uint32_t d = tmem_base + t * BN;
 #pragma unroll
         for (int kb = 0; kb < QK_UNITS; ++kb) {
@@ -200,6 +203,7 @@ mla_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       // O_t (+)= P_t V_j: P (bf16 pairs) occupies the first 64 columns of the score tile, 16 key
       // rows = 8 columns per step; V unit = 64 key rows, 16 rows = 2048 bytes per step
       auto issue_pv = [&](int t, int j, bool accumulate) {
+        if (!issuer) return;
         const uint32_t d = tmem_base + 2 * BN + t * DV;
         const uint32_t pt = tmem_base + t * BN;
 #pragma unroll
@@ -210,7 +214,7 @@ mla_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         }
         umma_commit(&pv_done[t]);
       };
-      ok = mbar_wait_bounded(q_full, 0, abort_flag, p.status, kTimeoutFullBarrier, blockIdx.x);
+      ok = mbar_wait_warp(q_full, 0, abort_flag, p.status, kTimeoutFullBarrier, blockIdx.x);
       if (ok) ok = wait_units(0, QK_UNITS);
       if (ok) {
         tc_fence_after();
@@ -225,7 +229,7 @@ mla_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         bool k_next = false;
         for (int t = 0; t < 2 && ok; ++t) {
           if (j < nt[t]) {
-            ok = mbar_wait_bounded(&p_full[t], j & 1, abort_flag, p.status, kTimeoutTmemFull, blockIdx.x);
+            ok = mbar_wait_warp(&p_full[t], j & 1, abort_flag, p.status, kTimeoutTmemFull, blockIdx.x);
             if (!ok) break;
             tc_fence_after();
             issue_pv(t, j, j > 0);
@@ -244,7 +248,7 @@ mla_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         free_units(j * KV_UNITS + QK_UNITS, V_UNITS);                       // V_j
         if (j + 1 < n_kv) free_units((j + 1) * KV_UNITS, QK_UNITS);         // K_{j+1}: both S_t issued above
       }
-      if (!ok) {
+      if (!ok && issuer) {
         umma_commit(drain_bar);
         const uint64_t t0 = globaltimer_ns();
         while (!mbar_try_wait(drain_bar, 0) && globaltimer_ns() - t0 < 100000000ull) {}

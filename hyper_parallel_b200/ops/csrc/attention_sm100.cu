@@ -19,6 +19,11 @@
 // swizzle, rows contiguous by 128 B -- the layout serves as K-major operand (Q, K, P) and as
 // MN-major operand (V) alike.
 //
+// The MMA issuer of all attention kernels is a whole warp that walks its loop in step, one elected lane
+// issuing: descriptors then stay in uniform registers.  Issued from a one-lane branch a product took some 75
+// cycles, more than the 32-64 tensor cycles of most of them: B=1, S=8192, 32/8 heads forward 512 -> 463 us,
+// backward 1763 -> 1585 us; MLA, S=4096, 128 heads, forward 772 -> 692 us, backward 2857 -> 2420 us.
+//
 // Every wait is bounded; on expiry a status code is recorded and all roles unwind.
 #include "attention_common.cuh"
 
@@ -77,7 +82,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(drain_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform(threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
 
   // heavy (late) query blocks first: they have the most key tiles under a causal mask
@@ -116,7 +121,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_base_slot;
+  const uint32_t tmem_base = uniform(*tmem_base_slot);
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer --
@@ -159,14 +164,15 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------- MMA issuer --
-    if (lane == 0 && n_kv > 0) {
+    if (n_kv > 0) {      // the whole warp walks the loop, one elected lane issues
+      const bool issuer = elect_one();
       constexpr uint32_t idesc_s = make_idesc(1, 1, 0, 0, BM, BN);   // Q (K-major) x K (K-major)
       constexpr uint32_t idesc_o = make_idesc(1, 1, 0, 1, BM, HD);   // P (K-major) x V (MN-major)
-      const uint32_t q_addr = smem_u32(sQ), kv_addr = smem_u32(sKV), p_addr = smem_u32(sP);
+      const uint32_t q_addr = uniform(smem_u32(sQ)), kv_addr = uniform(smem_u32(sKV)), p_addr = uniform(smem_u32(sP));
       const int nt[2] = {n0, n1};
       bool ok = true;
       auto wait_kv = [&](int idx) {
-        return mbar_wait_bounded(&kv_full[idx % KV_STAGES], (idx / KV_STAGES) & 1, abort_flag, p.status,
+        return mbar_wait_warp(&kv_full[idx % KV_STAGES], (idx / KV_STAGES) & 1, abort_flag, p.status,
                                  kTimeoutFullBarrier, blockIdx.x);
       };
       const uint64_t q_desc = make_smem_desc_sw128(q_addr, 0, 1024);
@@ -174,6 +180,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       const uint64_t v_desc = make_smem_desc_sw128(kv_addr, HALF_BYTES, 1024);   // V tile, MN-major
       const uint64_t p_desc = make_smem_desc_sw128(p_addr, 0, 1024);
       auto issue_s = [&](int t, int idx) {
+        if (!issuer) return;
         const uint64_t qa = desc_at(q_desc, t * TILE_BYTES);
         const uint64_t ka = desc_at(k_desc, (idx % KV_STAGES) * TILE_BYTES);
         const uint32_t d = tmem_base + t * BN;
@@ -186,6 +193,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         umma_commit(&s_full[t]);
       };
       auto issue_pv = [&](int t, int idx, bool accumulate) {
+        if (!issuer) return;
         // P: kv index is the contraction (64-wide halves, +32 B per 16); V: 16 kv rows = 2048 B,
         // the two 64-wide halves of the head dimension are HALF_BYTES apart (leading offset)
         const uint64_t va = desc_at(v_desc, (idx % KV_STAGES) * TILE_BYTES);
@@ -205,13 +213,13 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         }
         umma_commit(&pv_done[t]);
       };
-      ok = mbar_wait_bounded(q_full, 0, abort_flag, p.status, kTimeoutFullBarrier, blockIdx.x);
+      ok = mbar_wait_warp(q_full, 0, abort_flag, p.status, kTimeoutFullBarrier, blockIdx.x);
       if (ok) ok = wait_kv(0);
       if (ok) {
         tc_fence_after();
         for (int t = 0; t < 2; ++t)
           if (nt[t] > 0) issue_s(t, 0);
-        umma_commit(&kv_empty[0]);                           // K_0 is free once both S_t(K_0) retire
+        if (issuer) umma_commit(&kv_empty[0]);                           // K_0 is free once both S_t(K_0) retire
       }
       for (int j = 0; j < n_kv && ok; ++j) {
         ok = wait_kv(2 * j + 1);                      // V_j
@@ -220,7 +228,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         tc_fence_after();
         for (int t = 0; t < 2 && ok; ++t) {
           if (j < nt[t]) {
-            ok = mbar_wait_bounded(&p_full[t], j & 1, abort_flag, p.status, kTimeoutTmemFull, blockIdx.x);
+            ok = mbar_wait_warp(&p_full[t], j & 1, abort_flag, p.status, kTimeoutTmemFull, blockIdx.x);
             if (!ok) break;
             tc_fence_after();
             issue_pv(t, 2 * j + 1, j > 0);
@@ -228,10 +236,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
           if (j + 1 < nt[t]) issue_s(t, 2 * j + 2);
         }
         if (!ok) break;
-        umma_commit(&kv_empty[(2 * j + 1) % KV_STAGES]);                      // V_j
-        if (j + 1 < n_kv) umma_commit(&kv_empty[(2 * j + 2) % KV_STAGES]);    // K_{j+1}: both S_t issued above
+        if (issuer) umma_commit(&kv_empty[(2 * j + 1) % KV_STAGES]);                      // V_j
+        if (issuer && j + 1 < n_kv) umma_commit(&kv_empty[(2 * j + 2) % KV_STAGES]);    // K_{j+1}: both S_t issued above
       }
-      if (!ok) {
+      if (!ok && issuer) {
         umma_commit(drain_bar);
         const uint64_t t0 = globaltimer_ns();
         while (!mbar_try_wait(drain_bar, 0) && globaltimer_ns() - t0 < 100000000ull) {}
@@ -466,7 +474,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(drain_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform(threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   // (batch, kv head) pairs are processed in groups of `head_group`: the CTAs that run at the same
   // time then add into a few MB of the fp32 dQ (and re-read the same Q / dO), which stays in L2;
@@ -522,7 +530,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_base_slot;
+  const uint32_t tmem_base = uniform(*tmem_base_slot);
   // tensor-memory columns
   constexpr uint32_t COL_ST = 0;      // 2 x 64   (S^T, later dQ^T)
   constexpr uint32_t COL_DPT = 128;   // 2 x 64
@@ -571,12 +579,13 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------- MMA issuer --
-    if (lane == 0 && n_it > 0) {
+    if (n_it > 0) {      // the whole warp walks the loop, one elected lane issues
+      const bool issuer = elect_one();
       constexpr uint32_t idesc_st = make_idesc(1, 1, 0, 0, BN, BQ);    // K (K-major) x Q (K-major)
       constexpr uint32_t idesc_acc = make_idesc(1, 1, 0, 1, BN, HD);   // P^T (K-major) x dO (MN-major)
       constexpr uint32_t idesc_dq = make_idesc(1, 1, 1, 1, HD, BQ);    // K^T (MN-major) x dS^T (MN-major)
-      const uint32_t k_addr = smem_u32(sK), v_addr = smem_u32(sV), qdo_addr = smem_u32(sQdO),
-                     ds_addr = smem_u32(sDS);
+      const uint32_t k_addr = uniform(smem_u32(sK)), v_addr = uniform(smem_u32(sV)),
+                     qdo_addr = uniform(smem_u32(sQdO)), ds_addr = uniform(smem_u32(sDS));
       bool ok = true;
       const uint64_t k_desc = make_smem_desc_sw128(k_addr, 0, 1024);              // K as K-major A
       const uint64_t v_desc = make_smem_desc_sw128(v_addr, 0, 1024);              // V as K-major A
@@ -587,6 +596,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       const uint64_t dsm_desc = make_smem_desc_sw128(ds_addr, PT_BYTES, 1024);    // dS^T as MN-major B
       // S^T(it) and dP^T(it) into buffer it & 1 (st_full follows the S^T product, issued last)
       auto issue_dpt = [&](int it) {
+        if (!issuer) return;
         const int b = it & 1;
         const uint64_t doa = desc_at(qk_desc, (it % QDO_STAGES) * 2 * QTILE_BYTES + QTILE_BYTES);
 #pragma unroll
@@ -597,6 +607,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
                      desc_at(doa, kb * (QTILE_BYTES / 2) + kk * 32), idesc_st, (kb | kk) ? 1u : 0u);
       };
       auto issue_st = [&](int it) {
+        if (!issuer) return;
         const int b = it & 1;
         const uint64_t qa = desc_at(qk_desc, (it % QDO_STAGES) * 2 * QTILE_BYTES);
 #pragma unroll
@@ -608,10 +619,10 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         umma_commit(&st_full[b]);
       };
       auto wait_qdo = [&](int it) {
-        return mbar_wait_bounded(&qdo_full[it % QDO_STAGES], (it / QDO_STAGES) & 1, abort_flag, p.status,
+        return mbar_wait_warp(&qdo_full[it % QDO_STAGES], (it / QDO_STAGES) & 1, abort_flag, p.status,
                                  kTimeoutFullBarrier, blockIdx.x);
       };
-      ok = mbar_wait_bounded(kv_full, 0, abort_flag, p.status, kTimeoutFullBarrier, blockIdx.x);
+      ok = mbar_wait_warp(kv_full, 0, abort_flag, p.status, kTimeoutFullBarrier, blockIdx.x);
       for (int it = 0; it < 2 && it < n_it && ok; ++it) {
         ok = wait_qdo(it);
         if (ok) {
@@ -627,7 +638,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       for (int it = 0; it < n_it && ok; ++it) {
         const int b = it & 1;
         const uint32_t par = (it >> 1) & 1;
-        ok = mbar_wait_bounded(&ds_full[b], par, abort_flag, p.status, kTimeoutTmemFull, blockIdx.x);
+        ok = mbar_wait_warp(&ds_full[b], par, abort_flag, p.status, kTimeoutTmemFull, blockIdx.x);
         if (!ok) break;
         tc_fence_after();
         const uint64_t qa = desc_at(qm_desc, (it % QDO_STAGES) * 2 * QTILE_BYTES);
@@ -635,37 +646,39 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         const uint64_t dsa = desc_at(dsk_desc, b * PT_BYTES);
         const uint64_t dsm = desc_at(dsm_desc, b * PT_BYTES);
         const uint32_t first = it ? 1u : 0u;
-        // dQ^T = K^T dS^T  (contraction over the 128 key rows: 8 steps of 16) into the S^T buffer
+        if (issuer) {
+          // dQ^T = K^T dS^T  (contraction over the 128 key rows: 8 steps of 16) into the S^T buffer
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          umma_f16(tmem_base + COL_ST + b * BQ, desc_at(kt_desc, kk * 2048), desc_at(dsm, kk * 2048), idesc_dq,
-                   kk ? 1u : 0u);
-        umma_commit(&dq_full[b]);
-        // dV += P^T dO ; dK += dS^T Q   (contraction over the 64 query rows: 4 steps of 16).  P^T lies
-        // in the dP^T buffer of the step: query rows 0..31 in columns 0..15, 32..63 in columns 32..47
+          for (int kk = 0; kk < 8; ++kk)
+            umma_f16(tmem_base + COL_ST + b * BQ, desc_at(kt_desc, kk * 2048), desc_at(dsm, kk * 2048), idesc_dq,
+                     kk ? 1u : 0u);
+          umma_commit(&dq_full[b]);
+          // dV += P^T dO ; dK += dS^T Q   (contraction over the 64 query rows: 4 steps of 16).  P^T lies
+          // in the dP^T buffer of the step: query rows 0..31 in columns 0..15, 32..63 in columns 32..47
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-          umma_f16_ts(tmem_base + COL_DV, tmem_base + COL_DPT + b * BQ + (kk >> 1) * 32 + (kk & 1) * 8,
-                      desc_at(doa, kk * 2048), idesc_acc, kk ? 1u : first);
-        umma_f16(tmem_base + COL_DK, dsa, qa, idesc_acc, first);
+          for (int kk = 0; kk < 4; ++kk)
+            umma_f16_ts(tmem_base + COL_DV, tmem_base + COL_DPT + b * BQ + (kk >> 1) * 32 + (kk & 1) * 8,
+                        desc_at(doa, kk * 2048), idesc_acc, kk ? 1u : first);
+          umma_f16(tmem_base + COL_DK, dsa, qa, idesc_acc, first);
 #pragma unroll
-        for (int kk = 1; kk < 4; ++kk)
-          umma_f16(tmem_base + COL_DK, desc_at(dsa, kk * 32), desc_at(qa, kk * 2048), idesc_acc, 1u);
-        umma_commit(&qdo_empty[it % QDO_STAGES]);
-        umma_commit(&pt_free[b]);      // every reader of dS^T of this step has been issued
+          for (int kk = 1; kk < 4; ++kk)
+            umma_f16(tmem_base + COL_DK, desc_at(dsa, kk * 32), desc_at(qa, kk * 2048), idesc_acc, 1u);
+          umma_commit(&qdo_empty[it % QDO_STAGES]);
+          umma_commit(&pt_free[b]);      // every reader of dS^T of this step has been issued
+        }
         if (it + 2 < n_it) {
           ok = wait_qdo(it + 2);
           if (!ok) break;
           tc_fence_after();
           issue_dpt(it + 2);
-          ok = mbar_wait_bounded(&dq_drained[b], par, abort_flag, p.status, kTimeoutTmemEmpty, blockIdx.x);
+          ok = mbar_wait_warp(&dq_drained[b], par, abort_flag, p.status, kTimeoutTmemEmpty, blockIdx.x);
           if (!ok) break;
           tc_fence_after();
           issue_st(it + 2);
         }
       }
-      if (ok) umma_commit(acc_full);
-      if (!ok) {
+      if (ok && issuer) umma_commit(acc_full);
+      if (!ok && issuer) {
         umma_commit(drain_bar);
         const uint64_t t0 = globaltimer_ns();
         while (!mbar_try_wait(drain_bar, 0) && globaltimer_ns() - t0 < 100000000ull) {}

@@ -83,13 +83,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
       : "r"(taddr)
       : "memory");
 }
-// Bounded wait of a whole warp; every lane gets the same answer (a warp-uniform loop: the compiler can
-// then keep descriptors in uniform registers, an MMA issues in some 25 instead of 75 cycles).
-__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status,
-                                               int code, int detail) {
-  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
-  return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort_flag, status, code, detail));
-}
 __device__ __forceinline__ void cp_async4(float* dst, const float* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
@@ -114,7 +107,7 @@ gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
   uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(drain_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
 
-  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int num_m = (p.M + TILE_M - 1) / TILE_M, num_n = (p.N + TILE_N - 1) / TILE_N;
   const int num_tiles = num_m * num_n;
   const int num_k = p.K / BK;
@@ -190,10 +183,10 @@ gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     if (warp == 1) {
       // the whole warp walks the loop, one elected lane issues
       constexpr uint32_t idesc = make_idesc(0, 0, 0, 0, TILE_M, TILE_N);      // e4m3 x e4m3 -> fp32
-      const uint32_t base = __shfl_sync(0xffffffffu, smem_u32(smem), 0);
+      const uint32_t base = uniform(smem_u32(smem));
       const uint64_t a_desc = make_smem_desc_sw128(base, 0, 1024);
       const uint64_t b_desc = make_smem_desc_sw128(base + A_BYTES, 0, 1024);
-      const uint32_t tbase = __shfl_sync(0xffffffffu, tmem_base, 0);
+      const uint32_t tbase = uniform(tmem_base);
       const bool issuer = elect_one();
       int stage = 0, buf = 0;
       uint32_t phase = 0, bphase = 0;
