@@ -133,11 +133,11 @@ def flash_attention_backward(q, k, v, out, lse, do, causal: bool = True, scale: 
         dv = torch.empty((B, S, Hkv, D), dtype=torch.bfloat16, device=dev)
         dq_stride, dkv_stride = H * D, Hkv * D
     dq_acc = torch.empty((B, S, H, D), dtype=torch.float32, device=dev)
-    delta = torch.empty((B, H, S), dtype=torch.float32, device=dev)
+    stats = torch.empty((2, B, H, S), dtype=torch.float32, device=dev)
     rc = lib.hpb_flash_attn_bwd(q.data_ptr(), q.stride(0), q.stride(1), k.data_ptr(), k.stride(0), k.stride(1),
                                 v.data_ptr(), v.stride(0), v.stride(1), out.data_ptr(), lse.data_ptr(),
                                 do.data_ptr(), do.stride(0), do.stride(1), dq.data_ptr(), dk.data_ptr(),
-                                dv.data_ptr(), dq_stride, dkv_stride, dq_acc.data_ptr(), delta.data_ptr(), B, S, H,
+                                dv.data_ptr(), dq_stride, dkv_stride, dq_acc.data_ptr(), stats.data_ptr(), B, S, H,
                                 Hkv, float(scale if scale is not None else 1.0 / math.sqrt(D)), int(causal),
                                 native.status_word(dev).data_ptr(), native.stream(dev))
     native.check(rc, "hpb_flash_attn_bwd")

@@ -24,7 +24,7 @@
 //     i + 2 is formed while step i + 1 is still being exponentiated;
 //   * P^T (bf16 pairs) goes back into tensor memory, over the dP^T columns that the same thread has
 //     just read, and is the A operand of the dV product from there; only dS^T goes through shared
-//     memory (it is also a B operand), double buffered and handed back by the tensor core;
+//     memory (it is also a B operand), double buffered; the commit behind S^T(i + 2) hands it back;
 //   * per step the tensor core runs dV(i), dP^T(i + 1) (the softmax of step i + 1 waits for it;
 //     in-order execution keeps it behind the read of P^T), dK(i), the upper dQ^T(i) into the S^T
 //     buffer (the scores of step i + 1 are in registers by then), the lower dQ^T(i) while that
@@ -62,7 +62,7 @@ constexpr int PT_BYTES = BN * BQ * 2;           // 16 KB
 constexpr int BWD_THREADS = 448;
 constexpr int STAGE_TILE = BQ * 32 * 4;          // 8 KB: [64 query rows x 32 head elements] fp32
 constexpr int BWD_SMEM = 3 * UNIT_BYTES + 2 * UNIT_BYTES + RING * (Q_BYTES + DO_BYTES) + 2 * PT_BYTES +
-                         4 * STAGE_TILE + 2 * 2 * BQ * 4 + 1024 + 256;
+                         4 * STAGE_TILE + RING * 2 * BQ * 4 + 1024 + 256;
 static_assert(BWD_SMEM <= 227 * 1024, "shared memory budget");
 
 struct BwdParams {
@@ -72,8 +72,7 @@ struct BwdParams {
   int head_group;        // (batch, head) pairs scheduled together
   int probe;             // timing probes (results are wrong): 1 = no dQ staging / reduce, 2 = no exponentials,
                          // 4 / 8 / 16 = the dQ^T / dK, dV / S^T, dP^T products are not issued
-  const float* lse;      // [B, H, S]
-  const float* delta;    // [B, H, S]  rowsum(dO o O)
+  const float* stats;    // [2][B, H, S]: lse * log2(e), rowsum(dO o O)
   __nv_bfloat16* dKV;    // [B, S, H, 256]: dK nope | dV
   __nv_bfloat16* dKR;    // [B, S, H, 64]: dK of the rotary columns, per head
   int* status;
@@ -93,8 +92,8 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   uint8_t* sDO = sQ + RING * Q_BYTES;                         // ring of dO tiles (2 x 8 KB each)
   uint8_t* sDS = sDO + RING * DO_BYTES;                       // dS^T, two buffers of 16 KB
   uint8_t* sStage = sDS + 2 * PT_BYTES;                       // dQ staging: one 8 KB tile per dQ warp
-  float* sStat = reinterpret_cast<float*>(sStage + 4 * STAGE_TILE);  // [2][2][64]: lse * log2e, delta
-  uint64_t* kv_full = reinterpret_cast<uint64_t*>(sStat + 2 * 2 * BQ);
+  float* sStat = reinterpret_cast<float*>(sStage + 4 * STAGE_TILE);  // [RING][2][64]: lse * log2e, delta
+  uint64_t* kv_full = reinterpret_cast<uint64_t*>(sStat + RING * 2 * BQ);
   uint64_t* q_full = kv_full + 1;                // [2]
   uint64_t* q_empty = q_full + RING;             // [2]
   uint64_t* do_full = q_empty + RING;            // [2]
@@ -103,13 +102,11 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   uint64_t* st_consumed = st_full + 1;           // [1]  S^T of a step is in registers (8 warp arrivals)
   uint64_t* dpt_full = st_consumed + 1;          // [1]  dP^T of a step complete
   uint64_t* ds_full = dpt_full + 1;              // [2]  P^T / dS^T written, dP^T read (8 warp arrivals)
-  uint64_t* pt_free = ds_full + 2;               // [2]  every product reading dS^T buffer b has retired
-  uint64_t* dq_lo_full = pt_free + 2;            // [1]
+  uint64_t* dq_lo_full = ds_full + 2;            // [1]
   uint64_t* dq_hi_full = dq_lo_full + 1;         // [1]
   uint64_t* dq_lo_drained = dq_hi_full + 1;      // [1]  (4 warp arrivals)
   uint64_t* dq_hi_drained = dq_lo_drained + 1;   // [1]  (2 warp arrivals)
-  uint64_t* stat_full = dq_hi_drained + 1;       // [2]  lse / delta of a step staged (4 warp arrivals)
-  uint64_t* acc_full = stat_full + 2;            // [1]
+  uint64_t* acc_full = dq_hi_drained + 1;        // [1]
   uint64_t* drain_bar = acc_full + 1;            // [1]
   uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(drain_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
@@ -140,16 +137,12 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
     for (int s = 0; s < RING; ++s) {
-      mbar_init(&q_full[s], 1);
+      mbar_init(&q_full[s], 1 + 32);     // tile bytes; the 32 lanes that copy the row statistics
       mbar_init(&q_empty[s], 1);
       mbar_init(&do_full[s], 1);
       mbar_init(&do_empty[s], 1);
     }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(&ds_full[b], 8);
-      mbar_init(&pt_free[b], 1);
-      mbar_init(&stat_full[b], 4);
-    }
+    for (int b = 0; b < 2; ++b) mbar_init(&ds_full[b], 8);
     mbar_init(st_full, 1);
     mbar_init(st_consumed, 8);
     mbar_init(dpt_full, 1);
@@ -192,43 +185,50 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         tma_load_3d(sV + h * UNIT_BYTES, &tmap_kv, kv_full, head * DKV + DV + h * 64, k0, batch);
       }
       tma_load_3d(sK + 2 * UNIT_BYTES, &tmap_kr, kv_full, 0, k0, batch);
-      int q_issued = 0, do_issued = 0;
-      bool ok = true;
-      for (int it = 0; it < n_it && ok; ++it) {
-        const int slot = it % RING;
-        const uint32_t phase = (it / RING) & 1;
-        const int q0 = (i_start + it) * BQ;
-        ok = mbar_wait_bounded(&q_empty[slot], phase ^ 1, abort_flag, p.status, kTimeoutEmptyBarrier, blockIdx.x);
-        if (!ok) break;
+    }
+    int q_issued = 0, do_issued = 0;
+    bool ok = true;
+    for (int it = 0; it < n_it && ok; ++it) {
+      const int slot = it % RING;
+      const uint32_t phase = (it / RING) & 1;
+      const int q0 = (i_start + it) * BQ;
+      ok = mbar_wait_warp(&q_empty[slot], phase ^ 1, abort_flag, p.status, kTimeoutEmptyBarrier, blockIdx.x);
+      if (!ok) break;
+      if (lane == 0) {
         mbar_arrive_expect_tx(&q_full[slot], Q_BYTES);
 #pragma unroll
         for (int h = 0; h < 3; ++h)
           tma_load_3d(sQ + slot * Q_BYTES + h * QSUB_BYTES, &tmap_q, &q_full[slot], head * DQK + h * 64, q0, batch);
-        ++q_issued;
-        ok = mbar_wait_bounded(&do_empty[slot], phase ^ 1, abort_flag, p.status, kTimeoutEmptyBarrier, blockIdx.x);
-        if (!ok) break;
+      }
+      fetch_stats(sStat + slot * 2 * BQ, p.stats, (static_cast<int64_t>(batch) * p.H + head) * p.S,
+                  static_cast<int64_t>(p.B) * p.H * p.S, q0, p.S, lane, &q_full[slot]);
+      ++q_issued;
+      ok = mbar_wait_warp(&do_empty[slot], phase ^ 1, abort_flag, p.status, kTimeoutEmptyBarrier, blockIdx.x);
+      if (!ok) break;
+      if (lane == 0) {
         mbar_arrive_expect_tx(&do_full[slot], DO_BYTES);
 #pragma unroll
         for (int h = 0; h < 2; ++h)
           tma_load_3d(sDO + slot * DO_BYTES + h * QSUB_BYTES, &tmap_do, &do_full[slot], head * DV + h * 64, q0, batch);
-        ++do_issued;
       }
-      if (!ok) {
-        // wait (bounded) for the copies already issued, so that none lands after the CTA exits
-        const uint64_t t0 = globaltimer_ns();
-        while (!mbar_try_wait(kv_full, 0) && globaltimer_ns() - t0 < 100000000ull) {}
-        for (int b = 1; b <= min(q_issued, RING); ++b) {
-          const int it = q_issued - b;
-          const uint64_t t1 = globaltimer_ns();
-          while (!mbar_try_wait(&q_full[it % RING], (it / RING) & 1) && globaltimer_ns() - t1 < 100000000ull) {}
-        }
-        for (int b = 1; b <= min(do_issued, RING); ++b) {
-          const int it = do_issued - b;
-          const uint64_t t1 = globaltimer_ns();
-          while (!mbar_try_wait(&do_full[it % RING], (it / RING) & 1) && globaltimer_ns() - t1 < 100000000ull) {}
-        }
+      ++do_issued;
+    }
+    if (!ok && lane == 0) {
+      // wait (bounded) for the copies already issued, so that none lands after the CTA exits
+      const uint64_t t0 = globaltimer_ns();
+      while (!mbar_try_wait(kv_full, 0) && globaltimer_ns() - t0 < 100000000ull) {}
+      for (int b = 1; b <= min(q_issued, RING); ++b) {
+        const int it = q_issued - b;
+        const uint64_t t1 = globaltimer_ns();
+        while (!mbar_try_wait(&q_full[it % RING], (it / RING) & 1) && globaltimer_ns() - t1 < 100000000ull) {}
+      }
+      for (int b = 1; b <= min(do_issued, RING); ++b) {
+        const int it = do_issued - b;
+        const uint64_t t1 = globaltimer_ns();
+        while (!mbar_try_wait(&do_full[it % RING], (it / RING) & 1) && globaltimer_ns() - t1 < 100000000ull) {}
       }
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
   } else if (warp == 1) {
     // ---------------------------------------------------------- MMA issuer --
     if (n_it > 0) {      // the whole warp walks the loop, one elected lane issues
@@ -370,7 +370,6 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         for (int kk = 0; kk < 8; ++kk)
           umma_f16(tmem_base + COL_DQ, desc_at(kt_desc, kk * 2048), desc_at(dsm, kk * 2048), idesc_dq, kk ? 1u : 0u);
         if (issuer) umma_commit(dq_lo_full);
-        if (issuer) umma_commit(&pt_free[b]);     // every reader of dS^T of this step has been issued
         tick(3);
         // The upper tile must have left the S^T buffer before anything else is written there: S^T of
         // step it + 2, or -- in the last two steps, where no score tile follows -- the upper tile of
@@ -404,20 +403,10 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     bool ok = true;
     if (wg < 2) {
       // ------------------------------------------------------ softmax / dS --
-      const int tid = threadIdx.x - 64;       // 0..255 over both softmax groups; 0..127 stage the statistics
       const int kv_row = k0 + row;
       const bool row_live = kv_row < p.S;
       const int sw = row & 7;
       const int c = wg;                       // this group's 32 query columns
-      auto load_stat = [&](int it) -> float {
-        // threads 0..63 fetch lse (scaled to log2), 64..127 fetch delta, of step `it`
-        if (it >= n_it || tid >= 128) return 0.f;
-        const int q = (i_start + it) * BQ + (tid & 63);
-        if (q >= p.S) return tid < 64 ? INFINITY : 0.f;
-        const int64_t off = (static_cast<int64_t>(batch) * p.H + head) * p.S + q;
-        return tid < 64 ? p.lse[off] : p.delta[off];     // raw: scaled when staged, a step later
-      };
-      float stat_next = load_stat(0);
       const bool prof = p.prof != nullptr && blockIdx.x == 0 && threadIdx.x == 64;
       long long acc[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
       long long tp = prof ? clock64() : 0;
@@ -430,21 +419,10 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       };
       for (int it = 0; it < n_it && ok; ++it) {
         const int b = it & 1;
-        const uint32_t par = (it >> 1) & 1;
-        float* stat = sStat + b * 2 * BQ;
-        // dS^T buffer b is free again (the products of step it - 2 that read it have retired); this
-        // also means that all eight softmax warps have finished step it - 2, so the statistics
-        // buffer b can be rewritten
-        ok = mbar_wait_bounded(&pt_free[b], par ^ 1, abort_flag, p.status, kTimeoutTmemEmpty, blockIdx.x);
-        if (!ok) break;
-        tick(0);
-        if (tid < 128) stat[tid] = tid < 64 ? stat_next * 1.4426950408889634f : stat_next;
-        stat_next = load_stat(it + 1);
-        __syncwarp();
-        if (lane == 0 && wg == 0) mbar_arrive(&stat_full[b]);
-        ok = mbar_wait_bounded(&stat_full[b], par, abort_flag, p.status, kTimeoutFullBarrier, blockIdx.x);
-        tick(1);
-        if (ok) ok = mbar_wait_bounded(st_full, it & 1, abort_flag, p.status, kTimeoutTmemFull, blockIdx.x);
+        // One wait for the scores, the row statistics and dS^T buffer b: S^T(it) was issued behind the barrier
+        // on which the statistics landed and behind every product of step it - 2.
+        const float* stat = sStat + (it % RING) * 2 * BQ;
+        ok = mbar_wait_bounded(st_full, it & 1, abort_flag, p.status, kTimeoutTmemFull, blockIdx.x);
         if (!ok) break;
         tick(2);
         tc_fence_after();
@@ -671,13 +649,13 @@ extern "C" void hpb_mla_attn_set_probe(int mask) { g_mla_bwd_probe = mask; }
 // Backward.  q [B, S, H, 192], kv [B, S, H, 256] (k_nope | v), kr [B, S, 64], O / dO [B, S, H, 128] bf16
 // with the innermost dimension contiguous and row (token) / batch strides in elements; lse from the
 // forward.  Outputs (contiguous bf16): dQ [B, S, H, 192], dKV [B, S, H, 256] (dK nope | dV), dKR
-// [B, S, 64] (summed over the heads).  Workspace: dq_acc fp32 [B, S, H, 192] (cleared here), delta
-// fp32 [B, H, S], dkr_heads bf16 [B, S, H, 64].
+// [B, S, 64] (summed over the heads).  Workspace: dq_acc fp32 [B, S, H, 192] (cleared here), stats
+// fp32 [2, B, H, S], dkr_heads bf16 [B, S, H, 64].
 extern "C" int hpb_mla_attn_bwd(const void* q, long long q_batch_stride, long long q_row_stride, const void* kv,
                                 long long kv_batch_stride, long long kv_row_stride, const void* kr,
                                 long long kr_batch_stride, long long kr_row_stride, const void* O, const float* lse,
                                 const void* dO, long long do_batch_stride, long long do_row_stride, void* dQ,
-                                void* dKV, void* dKR, float* dq_acc, float* delta, void* dkr_heads, int B, int S,
+                                void* dKV, void* dKR, float* dq_acc, float* stats, void* dkr_heads, int B, int S,
                                 int H, float softmax_scale, int causal, int* status, cudaStream_t stream) {
   if (B <= 0 || S <= 0) return 0;
   if (H <= 0) return -2;
@@ -724,14 +702,8 @@ extern "C" int hpb_mla_attn_bwd(const void* q, long long q_batch_stride, long lo
   const int64_t nq = static_cast<int64_t>(B) * S * H * mla::DQK;
   cudaError_t e = cudaMemsetAsync(dq_acc, 0, nq * sizeof(float), stream);
   if (e != cudaSuccess) return static_cast<int>(e);
-  {
-    const int64_t warps = static_cast<int64_t>(B) * S * H;
-    const int threads = 256;
-    const int64_t blocks = (warps * 32 + threads - 1) / threads;
-    fa::attn_delta_kernel<<<static_cast<unsigned>(blocks), threads, 0, stream>>>(
-        reinterpret_cast<const __nv_bfloat16*>(dO), do_batch_stride, do_row_stride,
-        reinterpret_cast<const __nv_bfloat16*>(O), delta, B, S, H);
-  }
+  fa::launch_attn_stats(reinterpret_cast<const __nv_bfloat16*>(dO), do_batch_stride, do_row_stride,
+                        reinterpret_cast<const __nv_bfloat16*>(O), lse, stats, B, S, H, stream);
   mla::BwdParams p;
   p.B = B; p.S = S; p.H = H;
   p.scale = softmax_scale;
@@ -740,8 +712,7 @@ extern "C" int hpb_mla_attn_bwd(const void* q, long long q_batch_stride, long lo
   p.head_group = g_mla_bwd_head_group > 0 ? g_mla_bwd_head_group : (1 << 30);
   p.probe = g_mla_bwd_probe;
   p.prof = g_mla_bwd_prof;
-  p.lse = lse;
-  p.delta = delta;
+  p.stats = stats;
   p.dKV = reinterpret_cast<__nv_bfloat16*>(dKV);
   p.dKR = reinterpret_cast<__nv_bfloat16*>(dkr_heads);
   p.status = status;

@@ -431,15 +431,14 @@ constexpr int PT_BYTES = BN * BQ * 2;         // 16 KB
 constexpr int BWD_THREADS = 448;
 constexpr int STAGE_TILE = BQ * 32 * 4;       // 8 KB: [64 query rows x 32 head elements] fp32
 constexpr int BWD_SMEM = 2 * TILE_BYTES + QDO_STAGES * 2 * QTILE_BYTES + 2 * PT_BYTES + 4 * STAGE_TILE +
-                         2 * 2 * BQ * 4 + 1024 + 256;
+                         QDO_STAGES * 2 * BQ * 4 + 1024 + 256;
 
 struct BwdParams {
   int B, S, Hq, Hkv;
   float scale, scale_log2;
   int causal;
   int head_group;      // (batch, kv head) pairs scheduled together
-  const float* lse;    // [B, Hq, S]
-  const float* delta;  // [B, Hq, S]  rowsum(dO o O)
+  const float* stats;  // [2][B, Hq, S]: lse * log2(e), rowsum(dO o O)
   float* dQ;           // [B, S, Hq, 128] fp32, zero-initialised
   __nv_bfloat16* dK;   // [B, S, Hkv, 128], token stride dkv_row_stride elements
   __nv_bfloat16* dV;   // likewise
@@ -459,17 +458,15 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   uint8_t* sQdO = sV + TILE_BYTES;                            // per stage: Q (16 KB) | dO (16 KB)
   uint8_t* sDS = sQdO + QDO_STAGES * 2 * QTILE_BYTES;         // dS^T, two buffers of 16 KB
   uint8_t* sStage = sDS + 2 * PT_BYTES;                       // dQ staging: one 8 KB tile per dQ warp
-  float* sStat = reinterpret_cast<float*>(sStage + 4 * STAGE_TILE);  // [2][2][64]: lse*log2e, delta
-  uint64_t* kv_full = reinterpret_cast<uint64_t*>(sStat + 2 * 2 * BQ);
+  float* sStat = reinterpret_cast<float*>(sStage + 4 * STAGE_TILE);  // [QDO_STAGES][2][64]: lse*log2e, delta
+  uint64_t* kv_full = reinterpret_cast<uint64_t*>(sStat + QDO_STAGES * 2 * BQ);
   uint64_t* qdo_full = kv_full + 1;              // [QDO_STAGES]
   uint64_t* qdo_empty = qdo_full + QDO_STAGES;   // [QDO_STAGES]
   uint64_t* st_full = qdo_empty + QDO_STAGES;    // [2]  S^T and dP^T of a step are complete
   uint64_t* ds_full = st_full + 2;               // [2]  P^T / dS^T written (4 warp arrivals)
-  uint64_t* pt_free = ds_full + 2;               // [2]  products reading dS^T buffer b retired
-  uint64_t* dq_full = pt_free + 2;               // [2]
+  uint64_t* dq_full = ds_full + 2;               // [2]
   uint64_t* dq_drained = dq_full + 2;            // [2]  (4 warp arrivals)
-  uint64_t* stat_full = dq_drained + 2;          // [2]  lse / delta of a step staged (4 warp arrivals)
-  uint64_t* acc_full = stat_full + 2;            // [1]
+  uint64_t* acc_full = dq_drained + 2;           // [1]
   uint64_t* drain_bar = acc_full + 1;            // [1]
   uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(drain_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
@@ -502,16 +499,14 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
     for (int s = 0; s < QDO_STAGES; ++s) {
-      mbar_init(&qdo_full[s], 1);
+      mbar_init(&qdo_full[s], 1 + 32);     // tile bytes; the 32 lanes that copy the row statistics
       mbar_init(&qdo_empty[s], 1);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&st_full[b], 1);
       mbar_init(&ds_full[b], 8);
-      mbar_init(&pt_free[b], 1);     // committed by the MMA issuer behind the last reader of dS^T
       mbar_init(&dq_full[b], 1);
       mbar_init(&dq_drained[b], 4);
-      mbar_init(&stat_full[b], 4);
     }
     mbar_init(acc_full, 1);
     mbar_init(drain_bar, 1);
@@ -546,17 +541,18 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         tma_load_3d(sK + h * HALF_BYTES, &tmap_k, kv_full, kv_head * HD + h * 64, k0, batch);
         tma_load_3d(sV + h * HALF_BYTES, &tmap_v, kv_full, kv_head * HD + h * 64, k0, batch);
       }
-      int issued = 0;
-      bool ok = true;
-      for (int it = 0; it < n_it && ok; ++it) {
-        const int stage = it % QDO_STAGES;
-        const uint32_t phase = (it / QDO_STAGES) & 1;
-        ok = mbar_wait_bounded(&qdo_empty[stage], phase ^ 1, abort_flag, p.status, kTimeoutEmptyBarrier,
-                               blockIdx.x);
-        if (!ok) break;
-        const int head = kv_head * group + it / per_head;
-        const int q0 = (i_start + it % per_head) * BQ;
-        uint8_t* dq = sQdO + stage * 2 * QTILE_BYTES;
+    }
+    int issued = 0;
+    bool ok = true;
+    for (int it = 0; it < n_it && ok; ++it) {
+      const int stage = it % QDO_STAGES;
+      const uint32_t phase = (it / QDO_STAGES) & 1;
+      ok = mbar_wait_warp(&qdo_empty[stage], phase ^ 1, abort_flag, p.status, kTimeoutEmptyBarrier, blockIdx.x);
+      if (!ok) break;
+      const int head = kv_head * group + it / per_head;
+      const int q0 = (i_start + it % per_head) * BQ;
+      uint8_t* dq = sQdO + stage * 2 * QTILE_BYTES;
+      if (lane == 0) {
         mbar_arrive_expect_tx(&qdo_full[stage], 2 * QTILE_BYTES);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -564,19 +560,22 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
           tma_load_3d(dq + QTILE_BYTES + h * (QTILE_BYTES / 2), &tmap_do, &qdo_full[stage], head * HD + h * 64,
                       q0, batch);
         }
-        ++issued;
       }
-      if (!ok) {
-        const uint64_t t0 = globaltimer_ns();
-        while (!mbar_try_wait(kv_full, 0) && globaltimer_ns() - t0 < 100000000ull) {}
-        for (int b = 1; b <= min(issued, QDO_STAGES); ++b) {
-          const int it = issued - b;
-          const uint64_t t1 = globaltimer_ns();
-          while (!mbar_try_wait(&qdo_full[it % QDO_STAGES], (it / QDO_STAGES) & 1) &&
-                 globaltimer_ns() - t1 < 100000000ull) {}
-        }
+      fetch_stats(sStat + stage * 2 * BQ, p.stats, (static_cast<int64_t>(batch) * p.Hq + head) * p.S,
+                  static_cast<int64_t>(p.B) * p.Hq * p.S, q0, p.S, lane, &qdo_full[stage]);
+      ++issued;
+    }
+    if (!ok && lane == 0) {
+      const uint64_t t0 = globaltimer_ns();
+      while (!mbar_try_wait(kv_full, 0) && globaltimer_ns() - t0 < 100000000ull) {}
+      for (int b = 1; b <= min(issued, QDO_STAGES); ++b) {
+        const int it = issued - b;
+        const uint64_t t1 = globaltimer_ns();
+        while (!mbar_try_wait(&qdo_full[it % QDO_STAGES], (it / QDO_STAGES) & 1) &&
+               globaltimer_ns() - t1 < 100000000ull) {}
       }
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
   } else if (warp == 1) {
     // ---------------------------------------------------------- MMA issuer --
     if (n_it > 0) {      // the whole warp walks the loop, one elected lane issues
@@ -664,7 +663,6 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
           for (int kk = 1; kk < 4; ++kk)
             umma_f16(tmem_base + COL_DK, desc_at(dsa, kk * 32), desc_at(qa, kk * 2048), idesc_acc, 1u);
           umma_commit(&qdo_empty[it % QDO_STAGES]);
-          umma_commit(&pt_free[b]);      // every reader of dS^T of this step has been issued
         }
         if (it + 2 < n_it) {
           ok = wait_qdo(it + 2);
@@ -692,35 +690,17 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     bool ok = true;
     if (wg < 2) {
       // ------------------------------------------------------ softmax / dS --
-      const int tid = threadIdx.x - 64;       // 0..255 over both softmax groups; 0..127 stage the statistics
       const int kv_row = k0 + row;
       const bool row_live = kv_row < p.S;
       const int sw = row & 7;
-      auto load_stat = [&](int it) -> float {
-        // threads 0..63 fetch lse (scaled to log2), 64..127 fetch delta, of step `it`
-        if (it >= n_it || tid >= 128) return 0.f;
-        const int head = kv_head * group + it / per_head;
-        const int q = (i_start + it % per_head) * BQ + (tid & 63);
-        if (q >= p.S) return tid < 64 ? INFINITY : 0.f;
-        const int64_t off = (static_cast<int64_t>(batch) * p.Hq + head) * p.S + q;
-        return tid < 64 ? p.lse[off] : p.delta[off];     // raw: scaled when staged, a step later
-      };
-      float stat_next = load_stat(0);
       for (int it = 0; it < n_it && ok; ++it) {
         const int b = it & 1;
         const uint32_t par = (it >> 1) & 1;
-        float* stat = sStat + b * 2 * BQ;
-        // dS^T buffer b is free again (the products of step it - 2 that read it have retired); this
-        // also means that all eight softmax warps have finished step it - 2, so the statistics
-        // buffer b can be rewritten
-        ok = mbar_wait_bounded(&pt_free[b], par ^ 1, abort_flag, p.status, kTimeoutTmemEmpty, blockIdx.x);
-        if (!ok) break;
-        if (tid < 128) stat[tid] = tid < 64 ? stat_next * 1.4426950408889634f : stat_next;
-        stat_next = load_stat(it + 1);
-        __syncwarp();
-        if (lane == 0 && wg == 0) mbar_arrive(&stat_full[b]);
-        ok = mbar_wait_bounded(&stat_full[b], par, abort_flag, p.status, kTimeoutFullBarrier, blockIdx.x);
-        if (ok) ok = mbar_wait_bounded(&st_full[b], par, abort_flag, p.status, kTimeoutTmemFull, blockIdx.x);
+        // One wait covers everything this step needs.  S^T(it) was issued behind the barrier on which the row
+        // statistics of the step landed, and behind every product of step it - 2, so that its commit also says
+        // that dS^T buffer b is free again.  (Waits are dear here: 200-400 cycles each, even when complete.)
+        const float* stat = sStat + (it % QDO_STAGES) * 2 * BQ;
+        ok = mbar_wait_bounded(&st_full[b], par, abort_flag, p.status, kTimeoutTmemFull, blockIdx.x);
         if (!ok) break;
         tc_fence_after();
         const int q0 = (i_start + it % per_head) * BQ;
@@ -915,13 +895,13 @@ extern "C" int hpb_flash_attn_fwd(const void* q, long long q_batch_stride, long 
 // Backward.  dO [B, S, Hq, 128] (strided like q), O / lse from the forward.  Outputs: dQ
 // [B, S, Hq, 128] bf16, dK / dV [B, S, Hkv, 128] bf16 with token strides dq_row_stride / dkv_row_stride
 // elements (so that they may be the three column ranges of one packed gradient).  Workspace: dq_acc fp32
-// [B, S, Hq, 128] and delta fp32 [B, Hq, S]; dq_acc is cleared here.
+// [B, S, Hq, 128] and stats fp32 [2, B, Hq, S]; dq_acc is cleared here.
 extern "C" int hpb_flash_attn_bwd(const void* q, long long q_batch_stride, long long q_row_stride, const void* k,
                                   long long k_batch_stride, long long k_row_stride, const void* v,
                                   long long v_batch_stride, long long v_row_stride, const void* O, const float* lse,
                                   const void* dO, long long do_batch_stride, long long do_row_stride, void* dQ,
                                   void* dK, void* dV, long long dq_row_stride, long long dkv_row_stride,
-                                  float* dq_acc, float* delta, int B, int S, int Hq, int Hkv, float softmax_scale,
+                                  float* dq_acc, float* stats, int B, int S, int Hq, int Hkv, float softmax_scale,
                                   int causal, int* status, cudaStream_t stream) {
   if (B <= 0 || S <= 0) return 0;
   if (Hq <= 0 || Hkv <= 0 || Hq % Hkv) return -2;
@@ -955,22 +935,15 @@ extern "C" int hpb_flash_attn_bwd(const void* q, long long q_batch_stride, long 
   const int64_t nq = static_cast<int64_t>(B) * S * Hq * fa::HD;
   cudaError_t e = cudaMemsetAsync(dq_acc, 0, nq * sizeof(float), stream);
   if (e != cudaSuccess) return static_cast<int>(e);
-  {
-    const int64_t warps = static_cast<int64_t>(B) * S * Hq;
-    const int threads = 256;
-    const int64_t blocks = (warps * 32 + threads - 1) / threads;
-    fa::attn_delta_kernel<<<static_cast<unsigned>(blocks), threads, 0, stream>>>(
-        reinterpret_cast<const __nv_bfloat16*>(dO), do_batch_stride, do_row_stride,
-        reinterpret_cast<const __nv_bfloat16*>(O), delta, B, S, Hq);
-  }
+  fa::launch_attn_stats(reinterpret_cast<const __nv_bfloat16*>(dO), do_batch_stride, do_row_stride,
+                        reinterpret_cast<const __nv_bfloat16*>(O), lse, stats, B, S, Hq, stream);
   fa::BwdParams p;
   p.B = B; p.S = S; p.Hq = Hq; p.Hkv = Hkv;
   p.scale = softmax_scale;
   p.scale_log2 = softmax_scale * 1.4426950408889634f;
   p.causal = causal;
   p.head_group = g_bwd_head_group > 0 ? g_bwd_head_group : (1 << 30);
-  p.lse = lse;
-  p.delta = delta;
+  p.stats = stats;
   p.dQ = dq_acc;
   p.dK = reinterpret_cast<__nv_bfloat16*>(dK);
   p.dV = reinterpret_cast<__nv_bfloat16*>(dV);

@@ -109,12 +109,12 @@ def mla_backward(q, kv, k_rope, out, lse, do, causal: bool = True, scale: Option
     dkv = torch.empty((B, S, H, DN + DV), dtype=torch.bfloat16, device=dev)
     dkr = torch.empty((B, S, DR), dtype=torch.bfloat16, device=dev)
     dq_acc = torch.empty((B, S, H, DN + DR), dtype=torch.float32, device=dev)
-    delta = torch.empty((B, H, S), dtype=torch.float32, device=dev)
+    stats = torch.empty((2, B, H, S), dtype=torch.float32, device=dev)
     dkr_heads = torch.empty((B, S, H, DR), dtype=torch.bfloat16, device=dev)
     rc = lib.hpb_mla_attn_bwd(q.data_ptr(), q.stride(0), q.stride(1), kv.data_ptr(), kv.stride(0), kv.stride(1),
                               k_rope.data_ptr(), k_rope.stride(0), k_rope.stride(1), out.data_ptr(), lse.data_ptr(),
                               do.data_ptr(), do.stride(0), do.stride(1), dq.data_ptr(), dkv.data_ptr(),
-                              dkr.data_ptr(), dq_acc.data_ptr(), delta.data_ptr(), dkr_heads.data_ptr(), B, S, H,
+                              dkr.data_ptr(), dq_acc.data_ptr(), stats.data_ptr(), dkr_heads.data_ptr(), B, S, H,
                               float(scale if scale is not None else 1.0 / math.sqrt(DN + DR)), int(causal),
                               native.status_word(dev).data_ptr(), native.stream(dev))
     native.check(rc, "hpb_mla_attn_bwd")
