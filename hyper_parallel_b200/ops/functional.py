@@ -70,11 +70,16 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         out.copy_(res.to(out.dtype))
         return out
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
-    if a.stride(-1) != 1 or (a.stride(0) % 8) or (a.data_ptr() % 16):
+    a_ptr, (lda, a_inner) = a.data_ptr(), a.stride()
+    if a_inner != 1 or lda % 8 or a_ptr % 16:
         a = a.contiguous()
-    if b.stride(-1) != 1 or (b.stride(0) % 8) or (b.data_ptr() % 16):
+        a_ptr, lda = a.data_ptr(), a.stride(0)
+    b_ptr, (ldb, b_inner) = b.data_ptr(), b.stride()
+    if b_inner != 1 or ldb % 8 or b_ptr % 16:
         b = b.contiguous()
-    assert out.stride(-1) == 1 and out.dtype in (torch.bfloat16, torch.float32)
+        b_ptr, ldb = b.data_ptr(), b.stride(0)
+    out_f32 = out.dtype == torch.float32
+    assert out.stride(-1) == 1 and (out_f32 or out.dtype == torch.bfloat16)
     if M == 0 or N == 0:
         return out
     if K == 0:
@@ -84,22 +89,21 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     dev = a.device
     lib = native.lib()
     # CTA-pair (256x256, cta_group::2) kernel for large problems, single-CTA 128x256 otherwise
-    use_pair = _PAIR_MODE == "1" or (_PAIR_MODE == "auto" and M >= 512 and N >= 512 and hasattr(lib, "hpb_gemm2_bf16"))
+    use_pair = _PAIR_MODE == "1" or (_PAIR_MODE == "auto" and M >= 512 and N >= 512)
     if (use_pair and _RIDE_PROVIDER is not None and out.dtype == torch.bfloat16 and (a_mn, b_mn) in _RIDE_ORDERS
             and (not accumulate or (a_mn and b_mn))):
         ride = _RIDE_PROVIDER(dev, 2.0 * M * N * K)
         if ride is not None:
             import ctypes
-            rc = lib.hpb_gemm2_gather(a.data_ptr(), int(a_mn), a.stride(0), b.data_ptr(), int(b_mn), b.stride(0),
+            rc = lib.hpb_gemm2_gather(a_ptr, int(a_mn), lda, b_ptr, int(b_mn), ldb,
                                       out.data_ptr(), out.stride(0), int(accumulate), M, N, K, None, 0,
                                       ctypes.byref(ride), 2_000_000_000, native.status_word(dev).data_ptr(),
                                       native.sm_count(dev), native.stream(dev))
             native.check(rc, "hpb_gemm2_gather")
             return out
     fn = lib.hpb_gemm2_bf16 if use_pair else lib.hpb_gemm_bf16
-    rc = fn(a.data_ptr(), int(a_mn), a.stride(0), b.data_ptr(), int(b_mn), b.stride(0),
-            out.data_ptr(), out.stride(0), int(out.dtype == torch.float32), int(accumulate),
-            M, N, K, native.status_word(dev).data_ptr(), native.sm_count(dev), native.stream(dev))
+    rc = fn(a_ptr, a_mn, lda, b_ptr, b_mn, ldb, out.data_ptr(), out.stride(0), out_f32, accumulate, M, N, K,
+            native.status_word(dev).data_ptr(), native.sm_count(dev), native.stream(dev))
     native.check(rc, "hpb_gemm2_bf16" if use_pair else "hpb_gemm_bf16")
     return out
 
