@@ -128,7 +128,7 @@ class MLA(nn.Module):
         # attention kernels as the up-projection left it (k_nope | v per head), the shared rotary key
         # as one vector per token -- no concatenation or expansion on either pass
         q = _lin(ops.rmsnorm(_lin(x, self.wq_a, f8), self.q_norm, c.norm_eps), self.wq_b, f8)
-        q = mla_ops.rope_tail_(q.view(T, nh, dn + dr), dr, seq_len, c.rope_theta)
+        q = mla_ops.rope_tail_packed_(q, nh, dr, seq_len, c.rope_theta)
         kv_a = _lin(x, self.wkv_a, f8)
         kv_c, k_rope = kv_a.split([c.kv_lora_rank, dr], dim=-1)
         k_rope = _rope_last(k_rope.contiguous().view(T, 1, dr), seq_len, c.rope_theta)

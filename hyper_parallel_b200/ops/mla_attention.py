@@ -178,3 +178,32 @@ def rope_tail_(x: torch.Tensor, dr: int, seq_len: int, theta: float) -> torch.Te
     place and return ``x``; differentiable (the input must not be needed by the op that produced it,
     which holds for a projection output)."""
     return _RopeTail.apply(x, dr, seq_len, theta)
+
+
+class _RopeTailPacked(torch.autograd.Function):
+    """``_RopeTail`` on the packed ``x[T, NH * D]`` itself.  Modifying a view in place makes autograd
+    re-base the history (``CopySlices``), whose backward copies the whole gradient three times and
+    clears one more: 0.4 of 8.4 ms of a DeepSeek-V3 attention layer on 4096 tokens."""
+
+    @staticmethod
+    def forward(ctx, x, num_heads, dr, seq_len, theta):
+        from . import functional as Fn
+        ctx.meta = (num_heads, dr, seq_len, theta)
+        ctx.mark_dirty(x)
+        heads = x.view(x.shape[0], num_heads, -1)
+        Fn.rope_(heads[..., heads.shape[-1] - dr:], seq_len, theta)
+        return x
+
+    @staticmethod
+    def backward(ctx, dy):
+        from . import functional as Fn
+        num_heads, dr, seq_len, theta = ctx.meta
+        dx = dy.clone(memory_format=torch.contiguous_format)
+        heads = dx.view(dx.shape[0], num_heads, -1)
+        Fn.rope_(heads[..., heads.shape[-1] - dr:], seq_len, theta, inverse=True)
+        return dx, None, None, None, None
+
+
+def rope_tail_packed_(x: torch.Tensor, num_heads: int, dr: int, seq_len: int, theta: float) -> torch.Tensor:
+    """``rope_tail_`` for a projection output ``x[T, num_heads * D]`` that is not a view."""
+    return _RopeTailPacked.apply(x, num_heads, dr, seq_len, theta)
