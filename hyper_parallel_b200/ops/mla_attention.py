@@ -190,7 +190,7 @@ class _RopeTailPacked(torch.autograd.Function):
         from . import functional as Fn
         ctx.meta = (num_heads, dr, seq_len, theta)
         ctx.mark_dirty(x)
-        heads = x.view(x.shape[0], num_heads, -1)
+        heads = x.view(x.shape[0], num_heads, x.shape[1] // num_heads)     # (-1 is ambiguous without tokens)
         Fn.rope_(heads[..., heads.shape[-1] - dr:], seq_len, theta)
         return x
 
@@ -199,7 +199,7 @@ class _RopeTailPacked(torch.autograd.Function):
         from . import functional as Fn
         num_heads, dr, seq_len, theta = ctx.meta
         dx = dy.clone(memory_format=torch.contiguous_format)
-        heads = dx.view(dx.shape[0], num_heads, -1)
+        heads = dx.view(dx.shape[0], num_heads, dx.shape[1] // num_heads)
         Fn.rope_(heads[..., heads.shape[-1] - dr:], seq_len, theta, inverse=True)
         return dx, None, None, None, None
 

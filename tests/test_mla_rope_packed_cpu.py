@@ -16,3 +16,10 @@ def test_packed_equals_view(T, NH, D, dr, S):
     ya.backward(dy)
     yb.backward(dy)
     assert torch.equal(a.grad, b.grad)
+
+
+def test_no_tokens():
+    x = torch.zeros(0, 3 * 48, requires_grad=True)
+    y = mla_attention.rope_tail_packed_(x * 1.0, 3, 16, 4, 10000.0)
+    y.backward(torch.zeros_like(y))
+    assert y.shape == (0, 144) and x.grad.shape == (0, 144)
