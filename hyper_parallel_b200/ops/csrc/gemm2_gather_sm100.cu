@@ -435,7 +435,7 @@ gemm2_gather_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         const int col = col0 + c * 32;
         if (row < p.M && col < p.N) {
           __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<int64_t>(row) * p.ldc + col;
-          if (col + 32 <= p.N && (p.ldc & 7) == 0) {
+          if (col + 32 <= p.N && rows_aligned16(p.C, p.ldc * 2)) {
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               uint4* d4 = reinterpret_cast<uint4*>(dst) + j;

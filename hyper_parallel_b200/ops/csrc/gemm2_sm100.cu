@@ -203,6 +203,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     // --------------------------------------------------------------- epilogue (both) --
     const int q = warp & 3;
     int local_tile = 0, flip = 0;
+    const bool vec_c = rows_aligned16(p.C, p.ldc * (OUT_F32 ? 4 : 2));
     bool ok = true;
     auto release = [&](int buf) {
       tc_fence_before();
@@ -240,7 +241,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         if (row < p.M && col < p.N) {
           if constexpr (OUT_F32) {
             float* dst = reinterpret_cast<float*>(p.C) + static_cast<int64_t>(row) * p.ldc + col;
-            if (col + 32 <= p.N && (p.ldc & 3) == 0) {
+            if (col + 32 <= p.N && vec_c) {
 #pragma unroll
               for (int j = 0; j < 8; ++j) {
                 float4 v = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
@@ -261,7 +262,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             }
           } else {
             __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<int64_t>(row) * p.ldc + col;
-            if (col + 32 <= p.N && (p.ldc & 7) == 0) {
+            if (col + 32 <= p.N && vec_c) {
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
                 uint4* d4 = reinterpret_cast<uint4*>(dst) + j;

@@ -225,7 +225,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       if (!ok) break;
       if (row < p.M) {
         __nv_bfloat16* dst = p.C + static_cast<long long>(row) * p.ldc + n0;
-        if (n0 + HN <= p.N && (p.ldc & 7) == 0) {
+        if (n0 + HN <= p.N && rows_aligned16(p.C, p.ldc * 2)) {
 #pragma unroll
           for (int j = 0; j < HN / 8; ++j) {
             uint4 v;

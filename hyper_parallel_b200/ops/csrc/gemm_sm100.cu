@@ -14,7 +14,8 @@
 //   warp 0    : TMA producer (one elected lane)
 //   warp 1    : TMEM allocator + tcgen05.mma issuer (one lane)
 //   warps 2-5 : epilogue, tcgen05.ld TMEM -> registers -> shared -> TMA store (epilogue_store.cuh);
-//               accumulating products and unaligned C take plain 16-byte loads / stores per row
+//               accumulating products take plain loads / stores per row, and so does C whose rows do not
+//               start on 16-byte boundaries (element by element)
 // The 512 TMEM columns hold two 128x256 fp32 accumulators, so the epilogue of
 // tile i overlaps the main loop of tile i+1.
 //
@@ -262,6 +263,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
     // --------------------------------------------------------- epilogue --
     const int q = warp & 3;  // TMEM lane quarter this warp may read
     int local_tile = 0, flip = 0;
+    const bool vec_c = rows_aligned16(p.C, p.ldc * (OUT_F32 ? 4 : 2));
     bool ok = true;
     for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++local_tile) {
       const TileInfo ti = tile_info(t, p);
@@ -301,7 +303,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
         if (row_local < p.M && col < p.N && ti.group >= 0) {
           if constexpr (OUT_F32) {
             float* dst = reinterpret_cast<float*>(p.C) + row * p.ldc + col;
-            if (col + 32 <= p.N && (p.ldc & 3) == 0) {
+            if (col + 32 <= p.N && vec_c) {
 #pragma unroll
               for (int j = 0; j < 8; ++j) {
                 float4 v = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
@@ -323,7 +325,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
           } else {
             __nv_bfloat16* dst =
                 reinterpret_cast<__nv_bfloat16*>(p.C) + row * p.ldc + col;
-            if (col + 32 <= p.N && (p.ldc & 7) == 0) {
+            if (col + 32 <= p.N && vec_c) {
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
                 uint4* d4 = reinterpret_cast<uint4*>(dst) + j;

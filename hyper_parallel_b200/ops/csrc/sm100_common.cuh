@@ -149,6 +149,10 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
   if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
   return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort_flag, status, code, detail));
 }
+// Every row of a matrix starts on a 16-byte boundary (16-byte accesses to its rows are allowed).
+__host__ __device__ __forceinline__ bool rows_aligned16(const void* base, int64_t row_bytes) {
+  return ((reinterpret_cast<uintptr_t>(base) | static_cast<uintptr_t>(row_bytes)) & 15) == 0;
+}
 // The warp's index and other warp-uniform values, in a form that the compiler knows to be uniform.
 __device__ __forceinline__ uint32_t uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
 

@@ -18,7 +18,8 @@ TOL = {torch.bfloat16: 2.0 ** -8, torch.float32: 1e-5}
 @pytest.mark.parametrize("M,N,K", [(1, 8, 8), (31, 40, 72), (33, 72, 64), (127, 264, 128), (129, 248, 200),
                                    (257, 520, 64), (300, 1000, 24)])
 # out is a window of a larger buffer: (columns in front of it, extra columns in a row)
-@pytest.mark.parametrize("front,extra", [(0, 0), (8, 24), (1, 2), (8, 1)])
+# ((1, 7), (6, 2): rows a multiple of 16 bytes apart whose first one is not on such a boundary)
+@pytest.mark.parametrize("front,extra", [(0, 0), (8, 24), (1, 2), (8, 1), (1, 7), (6, 2)])
 def test_store_window(pair, dtype, M, N, K, front, extra):
     gen = torch.Generator(device="cuda").manual_seed(M * N + K)
     a = torch.randn(M, K, device="cuda", generator=gen).to(torch.bfloat16)
@@ -36,3 +37,26 @@ def test_store_window(pair, dtype, M, N, K, front, extra):
     rest = buf.clone()
     rest[1:M + 1, front:front + N] = 7.0
     assert (rest == 7.0).all()                 # nothing outside the window was written
+
+
+@pytest.mark.parametrize("pair", ["0", "1"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("front,extra", [(0, 0), (1, 7), (6, 2), (3, 0)])
+def test_accumulate_window(pair, dtype, front, extra):
+    M, N, K = 257, 264, 72
+    gen = torch.Generator(device="cuda").manual_seed(front)
+    a = torch.randn(M, K, device="cuda", generator=gen).to(torch.bfloat16)
+    b = torch.randn(N, K, device="cuda", generator=gen).to(torch.bfloat16)
+    buf = torch.randn(M + 2, front + N + extra, device="cuda", generator=gen).to(dtype)
+    before = buf.clone()
+    out = buf[1:M + 1, front:front + N]
+    Fn.set_gemm_pair_mode(pair)
+    try:
+        Fn.gemm(a, b, out=out, accumulate=True)
+    finally:
+        Fn.set_gemm_pair_mode("auto")
+    native.check_status()
+    ref = before[1:M + 1, front:front + N].double() + a.double() @ b.double().t()
+    assert ((out.double() - ref).norm() / ref.norm()).item() < TOL[dtype]
+    before[1:M + 1, front:front + N] = out
+    assert torch.equal(buf, before)
