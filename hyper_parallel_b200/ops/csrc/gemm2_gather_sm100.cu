@@ -28,6 +28,7 @@
 // be co-resident.  The only cross-GPU wait is for the peers' "shard version" flag, which a rank
 // publishes when its optimizer step has rewritten its shard; nothing waits for a peer's kernel of
 // the same step.  All waits are bounded and report through the status word.
+#include "epilogue_store.cuh"
 #include "gemm2_pair.cuh"
 
 #include <stdlib.h>
@@ -459,11 +460,7 @@ gemm2_gather_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
               *d4 = v;
             }
           } else {
-            for (int j = 0; j < 32 && col + j < p.N; ++j) {
-              float v = __uint_as_float(r[j]);
-              if constexpr (ACCUM) v += __bfloat162float(dst[j]);
-              dst[j] = __float2bfloat16(v);
-            }
+            store_row32_elements<ACCUM>(dst, r, p.N - col);
           }
         }
       }

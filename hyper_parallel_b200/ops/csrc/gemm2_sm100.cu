@@ -254,11 +254,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                 *d4 = v;
               }
             } else {
-              for (int j = 0; j < 32 && col + j < p.N; ++j) {
-                float v = __uint_as_float(r[j]);
-                if constexpr (ACCUM) v += dst[j];
-                dst[j] = v;
-              }
+              store_row32_elements<ACCUM>(dst, r, p.N - col);
             }
           } else {
             __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<int64_t>(row) * p.ldc + col;
@@ -286,11 +282,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                 *d4 = v;
               }
             } else {
-              for (int j = 0; j < 32 && col + j < p.N; ++j) {
-                float v = __uint_as_float(r[j]);
-                if constexpr (ACCUM) v += __bfloat162float(dst[j]);
-                dst[j] = __float2bfloat16(v);
-              }
+              store_row32_elements<ACCUM>(dst, r, p.N - col);
             }
           }
         }

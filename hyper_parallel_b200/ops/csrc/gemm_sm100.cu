@@ -316,11 +316,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
                 *d4 = v;
               }
             } else {
-              for (int j = 0; j < 32 && col + j < p.N; ++j) {
-                float v = __uint_as_float(r[j]);
-                if constexpr (ACCUM) v += dst[j];
-                dst[j] = v;
-              }
+              store_row32_elements<ACCUM>(dst, r, p.N - col);
             }
           } else {
             __nv_bfloat16* dst =
@@ -349,11 +345,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
                 *d4 = v;
               }
             } else {
-              for (int j = 0; j < 32 && col + j < p.N; ++j) {
-                float v = __uint_as_float(r[j]);
-                if constexpr (ACCUM) v += __bfloat162float(dst[j]);
-                dst[j] = __float2bfloat16(v);
-              }
+              store_row32_elements<ACCUM>(dst, r, p.N - col);
             }
           }
         }

@@ -1,0 +1,21 @@
+"""What the compiler reports about the kernels that were built (the log that the build keeps)."""
+import re
+
+import pytest
+
+from hyper_parallel_b200.ops import build
+
+
+def _entries():
+    log = build.BUILD_DIR / "ptxas.log"
+    if not log.exists() or not build.is_current():
+        pytest.skip("the library has not been built from these sources")
+    return re.findall(r"Compiling entry function '(\S+)'.*?\n.*?\n\s+(\d+) bytes stack frame", log.read_text())
+
+
+def test_gemm_accumulators_stay_in_registers():
+    """A stack frame in a GEMM means that its epilogue indexes the accumulator row at run time, which
+    sends every tile through local memory."""
+    gemms = [(name, int(frame)) for name, frame in _entries() if re.search(r"gemm\w*_kernel", name)]
+    assert len(gemms) > 40
+    assert not [name for name, frame in gemms if frame]
