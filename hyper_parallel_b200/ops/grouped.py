@@ -52,7 +52,7 @@ def _grouped(a, a_mn, a_rows, b, b_mn, b_rows, out, M, N, K, mode, block_group, 
              accumulate=False):
     dev = a.device
     rc = _lib().hpb_gemm_bf16_grouped(
-        a.data_ptr(), int(a_mn), a.stride(0), a_rows, b.data_ptr(), int(b_mn), b.stride(0), b_rows,
+        a.data_ptr(), a_mn, a.stride(0), a_rows, b.data_ptr(), b_mn, b.stride(0), b_rows,
         out.data_ptr(), out.stride(-2), int(out.dtype == torch.float32), int(accumulate), M, N, K, mode,
         native.ptr(block_group), native.ptr(group_offsets), E, b_group_rows,
         native.status_word(dev).data_ptr(), native.sm_count(dev), native.stream(dev))
@@ -130,111 +130,173 @@ def _expert_rows(a, w, out, block_group, pad, w_mn):
     E, rows_b = w.shape[0], w.shape[1]
     M, K = a.shape
     N = out.shape[1]
-    if pad == _BLOCK_M:
-        return _grouped(a, False, M, w.view(E * rows_b, -1), w_mn, E * rows_b, out, M, N, K, 1, block_group, None, E,
-                        rows_b)
     dev = a.device
+    if pad == _BLOCK_M:
+        native.check(_lib().hpb_gemm_bf16_grouped(
+            a.data_ptr(), 0, a.stride(0), M, w.data_ptr(), w_mn, w.stride(1), E * rows_b, out.data_ptr(), out.stride(0),
+            0, 0, M, N, K, 1, block_group.data_ptr(), None, E, rows_b, native.status_word(dev).data_ptr(),
+            native.sm_count(dev), native.stream(dev)), "hpb_gemm_bf16_grouped")
+        return out
     native.check(_local_lib().hpb_gemm2_bf16_grouped(
-        a.data_ptr(), a.stride(0), M, w.data_ptr(), int(w_mn), w.stride(1), E * rows_b, out.data_ptr(), out.stride(0),
+        a.data_ptr(), a.stride(0), M, w.data_ptr(), w_mn, w.stride(1), E * rows_b, out.data_ptr(), out.stride(0),
         M, N, K, 1, block_group.data_ptr(), None, None, E, rows_b, native.status_word(dev).data_ptr(),
         native.sm_count(dev), native.stream(dev)), "hpb_gemm2_bf16_grouped")
     return out
 
 
-def _expert_wgrad(a, b, out, starts, ends):
+def _expert_wgrad(a, b, out, table):
     """``out[e] = a[rows of e].T @ b[rows of e]``."""
     E, M, N = out.shape
     dev = a.device
     native.check(_local_lib().hpb_gemm2_bf16_grouped(
         a.data_ptr(), a.stride(0), a.shape[0], b.data_ptr(), 1, b.stride(0), b.shape[0], out.data_ptr(), N, M, N, 0, 2,
-        None, starts.data_ptr(), ends.data_ptr(), E, 0, native.status_word(dev).data_ptr(), native.sm_count(dev),
+        None, table.data_ptr(), table.data_ptr() + 4 * E, E, 0, native.status_word(dev).data_ptr(), native.sm_count(dev),
         native.stream(dev)), "hpb_gemm2_bf16_grouped")
     return out
 
 
-class _LocalExperts(torch.autograd.Function):
-    """``y[t] = sum_j gate[t, j] * expert_{idx[t, j]}(x[t])`` with every expert on this GPU
-    (``moe_local.cu`` around the grouped GEMMs).  One read-back of the per-expert counts, which sizes
-    the padded layout and refuses expert ids out of range."""
+class _Plan:
+    """Rows of a call: which padded row every (token, slot) pair takes.  One read-back of the per-expert
+    counts, which sizes the layout and refuses expert ids out of range.
 
-    @staticmethod
-    def forward(ctx, x, gate, w_gate_up, w_down, idx):
+    ``table``  [E] group starts, [E] group ends, [E] counts, 1 word: an id was out of range
+    ``slots``  [rows / pad] expert of each row block, [rows] pair of each row (-1: padding), [pairs] row of
+               each pair
+    Both are handed to the kernels as addresses into them: a tensor view each would cost the host more
+    than the launch."""
+
+    def __init__(self, idx, num_experts):
         lib = _local_lib()
-        dev = x.device
+        dev = idx.device
         stream = native.stream(dev)
         T, k = idx.shape
-        E, F2, H = w_gate_up.shape
-        pairs = T * k
+        E, pairs = num_experts, T * k
         pad = 256 if pairs >= _PAIR_MIN_ROWS * E else _BLOCK_M
-        gate_f = gate.detach().to(torch.float32).contiguous()
         hist = torch.empty((pairs + 255) // 256 * E, dtype=torch.int32, device=dev)
-        table = torch.empty(3 * E + 1, dtype=torch.int32, device=dev)
-        starts, ends, counts = table[:E], table[E:2 * E], table[2 * E:]
-        native.check(lib.hpb_moe_count(idx.data_ptr(), hist.data_ptr(), counts.data_ptr(), starts.data_ptr(),
-                                       ends.data_ptr(), pairs, E, pad, stream), "hpb_moe_count")
-        *per_expert, bad = counts.tolist()
+        self.table = torch.empty(3 * E + 1, dtype=torch.int32, device=dev)
+        starts = self.table.data_ptr()
+        native.check(lib.hpb_moe_count(idx.data_ptr(), hist.data_ptr(), starts + 8 * E, starts, starts + 4 * E, pairs, E,
+                                       pad, stream), "hpb_moe_count")
+        *per_expert, bad = self.table[2 * E:].tolist()
         if bad:
             raise ValueError(f"expert ids must lie in [0, {E})")
         rows = sum((c + pad - 1) // pad * pad for c in per_expert)
-        slots = torch.empty(rows // pad + rows + pairs, dtype=torch.int32, device=dev)
-        block_group, row_pair, pos = slots.split([rows // pad, rows, pairs])
-        native.check(lib.hpb_moe_place(idx.data_ptr(), hist.data_ptr(), starts.data_ptr(), ends.data_ptr(),
-                                       block_group.data_ptr(), row_pair.data_ptr(), pos.data_ptr(), pairs, E, pad,
+        self.dims = (T, k, E, rows, pad)
+        self.slots = torch.empty(rows // pad + rows + pairs, dtype=torch.int32, device=dev)
+        native.check(lib.hpb_moe_place(idx.data_ptr(), hist.data_ptr(), starts, starts + 4 * E, self.slots.data_ptr(),
+                                       _row_pair(self.slots, self.dims), _pos(self.slots, self.dims), pairs, E, pad,
                                        stream), "hpb_moe_place")
+
+
+def _row_pair(slots, dims):
+    return slots.data_ptr() + 4 * (dims[3] // dims[4])
+
+
+def _pos(slots, dims):
+    return _row_pair(slots, dims) + 4 * dims[3]
+
+
+def _pos_tensor(slots, dims):
+    """The row of every (token, slot) pair, for tensor operations."""
+    T, k = dims[:2]
+    return slots[slots.shape[0] - T * k:].view(T, k).long()
+
+
+class _ExpertRows(torch.autograd.Function):
+    """``yp[row of (t, j)] = expert_{idx[t, j]}(x[t])`` in the padded layout of the grouped GEMMs."""
+
+    @staticmethod
+    def forward(ctx, x, w_gate_up, w_down, plan):
+        lib = _local_lib()
+        dev = x.device
+        stream = native.stream(dev)
+        T, k, E, rows, pad = plan.dims
+        _, F2, H = w_gate_up.shape
         xp = torch.empty((rows, H), dtype=x.dtype, device=dev)
-        native.check(lib.hpb_moe_gather(x.data_ptr(), row_pair.data_ptr(), xp.data_ptr(), rows, k, H, stream),
-                     "hpb_moe_gather")
+        native.check(lib.hpb_moe_gather(x.data_ptr(), _row_pair(plan.slots, plan.dims), xp.data_ptr(), rows, k, H,
+                                        stream), "hpb_moe_gather")
         gu = torch.empty((rows, F2), dtype=x.dtype, device=dev)
-        _expert_rows(xp, w_gate_up, gu, block_group, pad, False)
+        _expert_rows(xp, w_gate_up, gu, plan.slots, pad, False)
         act = torch.empty((rows, F2 // 2), dtype=x.dtype, device=dev)
         native.check(lib.hpb_swiglu_fwd(gu.data_ptr(), act.data_ptr(), rows, F2 // 2, native.sm_count(dev), stream),
                      "hpb_swiglu_fwd")
         yp = torch.empty((rows, H), dtype=x.dtype, device=dev)
-        _expert_rows(act, w_down, yp, block_group, pad, False)
-        y = torch.empty((T, H), dtype=x.dtype, device=dev)
-        native.check(lib.hpb_moe_combine(yp.data_ptr(), pos.data_ptr(), gate_f.data_ptr(), y.data_ptr(), T, k, H,
-                                         stream), "hpb_moe_combine")
-        ctx.save_for_backward(xp, gu, act, yp if ctx.needs_input_grad[1] else None, gate_f, w_gate_up, w_down, table,
-                              slots)
-        ctx.dims = (T, k, E, rows, pad)
-        ctx.gate_dtype = gate.dtype
-        return y
+        _expert_rows(act, w_down, yp, plan.slots, pad, False)
+        ctx.save_for_backward(xp, gu, act, w_gate_up, w_down, plan.table, plan.slots)
+        ctx.dims = plan.dims
+        return yp
 
     @staticmethod
-    def backward(ctx, dy):
-        xp, gu, act, yp, gate_f, w_gate_up, w_down, table, slots = ctx.saved_tensors
+    def backward(ctx, dyp):
+        xp, gu, act, w_gate_up, w_down, table, slots = ctx.saved_tensors
         T, k, E, rows, pad = ctx.dims
         lib = _local_lib()
         dev, dt = xp.device, xp.dtype
         stream = native.stream(dev)
         H, F2 = xp.shape[1], gu.shape[1]
-        block_group, row_pair, pos = slots.split([rows // pad, rows, T * k])
-        starts, ends = table[:E], table[E:2 * E]
-        need_x, need_gate, need_w1, need_w2 = ctx.needs_input_grad[:4]
-        dy = _rows16(dy)
-        dyp = torch.empty((rows, H), dtype=dt, device=dev)
-        dgate = torch.empty((T, k), dtype=torch.float32, device=dev) if need_gate else None
-        native.check(lib.hpb_moe_combine_bwd(dy.data_ptr(), row_pair.data_ptr(), gate_f.data_ptr(), native.ptr(yp),
-                                             dyp.data_ptr(), native.ptr(dgate), rows, k, H, stream),
-                     "hpb_moe_combine_bwd")
+        need_x, need_w1, need_w2 = ctx.needs_input_grad[:3]
+        dyp = _rows16(dyp)
         dx = dw1 = dw2 = None
         if need_w2:
-            dw2 = _expert_wgrad(dyp, act, torch.empty_like(w_down), starts, ends)
+            dw2 = _expert_wgrad(dyp, act, torch.empty_like(w_down), table)
         if need_x or need_w1:
             dact = torch.empty_like(act)
-            _expert_rows(dyp, w_down, dact, block_group, pad, True)
+            _expert_rows(dyp, w_down, dact, slots, pad, True)
             dgu = torch.empty_like(gu)
             native.check(lib.hpb_swiglu_bwd(gu.data_ptr(), dact.data_ptr(), dgu.data_ptr(), rows, F2 // 2,
                                             native.sm_count(dev), stream), "hpb_swiglu_bwd")
             if need_w1:
-                dw1 = _expert_wgrad(dgu, xp, torch.empty_like(w_gate_up), starts, ends)
+                dw1 = _expert_wgrad(dgu, xp, torch.empty_like(w_gate_up), table)
             if need_x:
                 dxp = torch.empty((rows, H), dtype=dt, device=dev)
-                _expert_rows(dgu, w_gate_up, dxp, block_group, pad, True)
+                _expert_rows(dgu, w_gate_up, dxp, slots, pad, True)
                 dx = torch.empty((T, H), dtype=dt, device=dev)
-                native.check(lib.hpb_moe_combine(dxp.data_ptr(), pos.data_ptr(), None, dx.data_ptr(), T, k, H, stream),
-                             "hpb_moe_combine")
-        return dx, dgate.to(ctx.gate_dtype) if need_gate else None, dw1, dw2, None
+                native.check(lib.hpb_moe_combine(dxp.data_ptr(), _pos(slots, ctx.dims), None, dx.data_ptr(), T, k, H,
+                                                 stream), "hpb_moe_combine")
+        return dx, dw1, dw2, None
+
+
+def _combine_rows(yp, gate, slots, dims):
+    T, k, _, _, _ = dims
+    y = torch.empty((T, yp.shape[1]), dtype=yp.dtype, device=yp.device)
+    native.check(_local_lib().hpb_moe_combine(yp.data_ptr(), _pos(slots, dims), gate.data_ptr(), y.data_ptr(), T, k,
+                                              yp.shape[1], native.stream(yp.device)), "hpb_moe_combine")
+    return y
+
+
+class _Combine(torch.autograd.Function):
+    """``y[t] = sum_j gate[t, j] * yp[row of (t, j)]``; ``gate`` fp32, contiguous.  A node of its own, so
+    that the gate weights keep their higher derivatives (the products of the experts have none)."""
+
+    @staticmethod
+    def forward(ctx, yp, gate, plan):
+        ctx.save_for_backward(yp if ctx.needs_input_grad[1] else None, gate, plan.slots)
+        ctx.dims, ctx.like = plan.dims, (yp.dtype, yp.shape[1])
+        return _combine_rows(yp, gate, plan.slots, plan.dims)
+
+    @staticmethod
+    def backward(ctx, dy):
+        yp, gate, slots = ctx.saved_tensors
+        T, k, _, rows, _ = ctx.dims
+        dtype, H = ctx.like
+        need_rows, need_gate = ctx.needs_input_grad[:2]
+        dyp = dgate = None
+        if torch.is_grad_enabled() or not torch._C._has_storage(dy):
+            # a graph of the gradients, or a batch of them, is wanted: the same sums as tensor operations
+            pos = _pos_tensor(slots, ctx.dims)
+            if need_rows:
+                dyp = torch.zeros((rows, H), dtype=dtype, device=dy.device).index_copy(
+                    0, pos.view(-1), (gate[:, :, None] * dy[:, None].float()).to(dtype).reshape(T * k, H))
+            if need_gate:
+                dgate = torch.stack([(dy.float() * yp.index_select(0, pos[:, j]).float()).sum(-1) for j in range(k)], -1)
+            return dyp, dgate, None
+        dy = _rows16(dy)
+        dyp = torch.empty((rows, H), dtype=dtype, device=dy.device)
+        dgate = torch.empty((T, k), dtype=torch.float32, device=dy.device) if need_gate else None
+        native.check(_local_lib().hpb_moe_combine_bwd(dy.data_ptr(), _row_pair(slots, ctx.dims), gate.data_ptr(),
+                                                      native.ptr(yp), dyp.data_ptr(), native.ptr(dgate), rows, k, H,
+                                                      native.stream(dy.device)), "hpb_moe_combine_bwd")
+        return dyp, dgate, None
 
 
 def _plain(t: torch.Tensor) -> bool:
@@ -253,7 +315,18 @@ def local_experts_usable(x, topk_idx, topk_w, w_gate_up, w_down, num_experts) ->
 
 
 def local_experts(x, topk_idx, topk_w, w_gate_up, w_down):
-    return _LocalExperts.apply(_rows16(x), topk_w, _rows16(w_gate_up), _rows16(w_down), topk_idx.contiguous())
+    """``y[t] = sum_j topk_w[t, j] * expert_{topk_idx[t, j]}(x[t])`` with every expert on this GPU
+    (``moe_local.cu`` around the grouped GEMMs)."""
+    plan = _Plan(topk_idx.contiguous(), w_gate_up.shape[0])
+    yp = _ExpertRows.apply(_rows16(x), _rows16(w_gate_up), _rows16(w_down), plan)
+    # a copy: a caller may overwrite its gate weights before the backward pass
+    gate = topk_w.to(torch.float32, copy=True, memory_format=torch.contiguous_format)
+    if torch.autograd.forward_ad.unpack_dual(gate).tangent is not None:
+        pos = _pos_tensor(plan.slots, plan.dims)
+        return sum(gate[:, j, None] * yp.index_select(0, pos[:, j]).float() for j in range(pos.shape[1])).to(x.dtype)
+    if not (torch.is_grad_enabled() and (yp.requires_grad or gate.requires_grad)):
+        return _combine_rows(yp, gate, plan.slots, plan.dims)
+    return _Combine.apply(yp, gate, plan)
 
 
 def _rows16(t: torch.Tensor) -> torch.Tensor:

@@ -102,3 +102,78 @@ def test_frozen_weights_and_inputs():
         moe.expert_parallel_ffn(leaves[0], idx, leaves[1], leaves[2], leaves[3], 4).backward(dy)
         assert [t.grad is not None for t in leaves] == [j == i for j in range(4)], name
         assert _err(leaves[i].grad, want[i + 1]) < TOL
+
+
+# ---- the gate weights are ordinary operands: higher derivatives, forward mode, batched gradients ----
+def _toy(requires):
+    x, idx, gate, w1, w2, dy = _inputs(23, 2, 4, 64, 16, "plain")
+    return [t.requires_grad_(n in requires) for t, n in zip((x, gate, w1, w2), "xgab")], idx, dy
+
+
+def _dense(x, idx, gate, w1, w2):
+    """The layer in 64 bits."""
+    xd, w1, w2 = x.double(), w1.double(), w2.double()
+    y = 0
+    for e in range(w1.shape[0]):
+        g, u = (xd @ w1[e].t()).chunk(2, -1)
+        y = y + (F.silu(g) * u) @ w2[e].t() * (gate.double() * (idx == e)).sum(-1, keepdim=True)
+    return y
+
+
+@pytest.mark.parametrize("requires", ["g", "xgab"])
+def test_second_derivative_of_the_gate(requires):
+    """A penalty on the gradient of the gate: its own derivatives, and those of the experts through one
+    more (first-order) backward pass."""
+    def penalty(fn, x, gate, w1, w2, idx):
+        y = fn(x, idx, gate, w1, w2).double()
+        (d,) = torch.autograd.grad((y * y).sum(), gate, create_graph=True)
+        return (d.double() ** 2).sum()
+    (x, gate, w1, w2), idx, _ = _toy(requires)
+    penalty(lambda x, i, g, a, b: moe.expert_parallel_ffn(x, i, g, a, b, 4), x, gate, w1, w2, idx).backward()
+    native.check_status()
+    ref = [t.detach().double().requires_grad_(t.requires_grad) for t in (x, gate, w1, w2)]
+    penalty(_dense, *ref, idx).backward()
+    assert _err(gate.grad, ref[1].grad) < TOL
+    if requires == "g":
+        return
+    # only the path through the gate's gradient has a graph (the experts' gradients do not): what the general
+    # formulation gives for the inputs and weights is the same partial sum
+    got = [t.grad.clone() for t in (x, w1, w2)]
+    for t in (x, gate, w1, w2):
+        t.grad = None
+    general = pytest.MonkeyPatch()
+    general.setattr(grouped, "local_experts_usable", lambda *a: False)
+    try:
+        penalty(lambda x, i, g, a, b: moe.expert_parallel_ffn(x, i, g, a, b, 4), x, gate, w1, w2, idx).backward()
+    finally:
+        general.undo()
+    for a, t in zip(got, (x, w1, w2)):
+        assert _err(a, t.grad) < 2 * TOL
+
+
+def test_forward_mode_through_the_gate():
+    (x, gate, w1, w2), idx, _ = _toy("")
+    t = torch.randn_like(gate)
+    with torch.autograd.forward_ad.dual_level():
+        y = moe.expert_parallel_ffn(x, idx, torch.autograd.forward_ad.make_dual(gate, t), w1, w2, 4)
+        primal, tangent = torch.autograd.forward_ad.unpack_dual(y)
+    assert _err(primal, _dense(x, idx, gate, w1, w2)) < TOL
+    assert _err(tangent, _dense(x, idx, t, w1, w2)) < TOL       # linear in the gate
+
+
+def test_batched_gradients_of_the_gate():
+    (x, gate, w1, w2), idx, dy = _toy("g")
+    y = moe.expert_parallel_ffn(x, idx, gate, w1, w2, 4)
+    dys = torch.stack([dy, -2 * dy])
+    (got,) = torch.autograd.grad(y, gate, dys, is_grads_batched=True, retain_graph=True)
+    (one,) = torch.autograd.grad(y, gate, dy)
+    assert _err(got[0], one) < 1e-5 and _err(got[1], -2 * one) < 1e-5
+
+
+def test_gate_overwritten_before_the_backward_pass():
+    (x, gate, w1, w2), idx, dy = _toy("xab")
+    want = _pass(moe.expert_parallel_ffn, x, idx, gate.clone(), w1, w2, dy)
+    y = moe.expert_parallel_ffn(x, idx, gate, w1, w2, 4)
+    gate.zero_()
+    y.backward(dy)
+    assert torch.equal(x.grad, want[1]) and torch.equal(w1.grad, want[3]) and torch.equal(w2.grad, want[4])
