@@ -305,11 +305,12 @@ def _plain(t: torch.Tensor) -> bool:
 
 def local_experts_usable(x, topk_idx, topk_w, w_gate_up, w_down, num_experts) -> bool:
     """Calls that ``local_experts`` serves; every other one takes the general formulation."""
-    return (x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 2 and all(map(_plain, (x, topk_w, w_gate_up, w_down)))
+    return (x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 2
+            and all(map(_plain, (x, topk_idx, topk_w, w_gate_up, w_down)))
             and w_gate_up.dtype == w_down.dtype == torch.bfloat16 and w_gate_up.dim() == 3 and w_down.dim() == 3
             and w_gate_up.device == w_down.device == topk_idx.device == topk_w.device == x.device
             and topk_w.is_floating_point() and topk_w.shape == topk_idx.shape and topk_idx.dtype == torch.int64
-            and topk_idx.shape[0] == x.shape[0] and topk_idx.numel() > 0 and w_gate_up.shape[0] == num_experts <= 8192
+            and topk_idx.shape[0] == x.shape[0] and 0 < topk_idx.numel() < 1 << 30 and w_gate_up.shape[0] == num_experts <= 8192
             and w_gate_up.shape[2] == x.shape[1] and w_gate_up.shape[1] % 16 == 0 and x.shape[1] % 8 == 0
             and w_down.shape == (num_experts, x.shape[1], w_gate_up.shape[1] // 2))
 

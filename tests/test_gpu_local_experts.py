@@ -177,3 +177,11 @@ def test_gate_overwritten_before_the_backward_pass():
     gate.zero_()
     y.backward(dy)
     assert torch.equal(x.grad, want[1]) and torch.equal(w1.grad, want[3]) and torch.equal(w2.grad, want[4])
+
+
+def test_calls_beyond_the_row_tables_take_the_general_path():
+    """2^30 pairs and more do not fit the 32-bit tables (expanded inputs: nothing is allocated)."""
+    x, idx, gate, w1, w2, _ = _inputs(1, 1, 2, 64, 16, "plain")
+    assert grouped.local_experts_usable(x, idx, gate, w1, w2, 2)
+    many = [t.expand(1 << 30, t.shape[1]) for t in (x, idx, gate)]
+    assert not grouped.local_experts_usable(*many, w1, w2, 2)
