@@ -293,9 +293,10 @@ quant_act_1x128_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict_
                        int K) {
   __shared__ float sc[2][QA_ROWS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kb0 = blockIdx.y * 2, kblocks = K / 128;
+  // (a grid's second dimension ends at 65535: 2^24 columns; the third goes on)
+  const int kb0 = (blockIdx.z * gridDim.y + blockIdx.y) * 2, kblocks = K / 128;
   const int col = kb0 * 128 + lane * 8;
-  const bool live = col < K;
+  const bool live = kb0 + (lane >> 4) < kblocks;
   const int r0 = blockIdx.x * QA_ROWS + warp * 4;
   uint4 v[4];
 #pragma unroll
@@ -425,8 +426,8 @@ extern "C" int hpb_quant_act_1x128(const void* x, void* q, float* scales, int M,
   if (K % 128 || M <= 0) return K % 128 ? -2 : 0;
   // (cudaMalloc'ed or whole-row pointers are 16-byte aligned; K % 128 keeps every vector so)
   if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(q) & 7)) return -2;
-  const dim3 grid((M + QA_ROWS - 1) / QA_ROWS, (K / 128 + 1) / 2);
-  if (grid.y > 65535) return -2;
+  const int pairs = (K / 128 + 1) / 2, planes = (pairs + 65534) / 65535;
+  const dim3 grid((M + QA_ROWS - 1) / QA_ROWS, (pairs + planes - 1) / planes, planes);
   quant_act_1x128_kernel<<<grid, 256, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<uint8_t*>(q),
                                               scales, M, K);
   return static_cast<int>(cudaGetLastError());

@@ -40,3 +40,12 @@ def test_quantisers(M, K, form):
         x[M // 2, :128] = 1e-30
     _same(fp8.quantize_act_1x128(x), _want(x.cpu(), 1))
     _same(fp8.quantize_weight_128x128(x), _want(x.cpu(), 128))
+
+
+def test_more_column_blocks_than_a_grid_has_rows():
+    """One row of 2^24 + 128 columns: 131073 blocks of columns (a grid's second dimension ends at 65535)."""
+    K = (1 << 24) + 128
+    x = torch.randn(1, K, device="cuda").to(torch.bfloat16)
+    q, s = fp8.quantize_act_1x128(x)
+    wq, ws = _want(x.cpu(), 1)
+    _same((q, s), (wq, ws))
