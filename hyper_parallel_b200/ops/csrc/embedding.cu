@@ -6,16 +6,16 @@
 // memory).  No sort over the tokens and no floating-point atomics:
 //
 //   1. count   cnt[v] += 1 per token (integer atomics: the result does not depend on the order)
-//   2. scan    off[v] = exclusive prefix sum of cnt over the vocabulary: sums of 1024 counts, then every
+//   2. scan    off[v] = exclusive prefix sum of cnt over the vocabulary: sums of 1024 counts, and every
 //              CTA adds up the sums in front of its 1024 and scans them (one CTA that walked the whole
 //              vocabulary took 280 us for 128256 rows; the two launches take 7)
 //   3. fill    bucket[off[v] + k] = t, k handed out by an integer atomic (order inside a bucket varies)
-//   4. sum     one CTA per vocabulary row and 256 of its vectors: the bucket is rank-sorted by token index
-//              in shared memory (token indices are distinct, buckets are short), then the rows are added in
-//              that order -- the same order, hence the same bits, on every run.  Buckets longer than
-//              kMaxSorted tokens are added in bucket order (still correct, order not fixed).  Bound by
-//              writing dW (238 us for 128256 x 4096 and 8192 Zipf-distributed tokens, 370 us before); a CTA fetches the counts of kSumRows rows at once, so that the many rows without a
-//              token cost no load latency each, and keeps eight rows of a long bucket in flight.
+//   4. sum     one CTA per one or two vocabulary rows and 256 of their vectors: the bucket is rank-sorted by
+//              token index in shared memory (token indices are distinct, buckets are short), then the rows are
+//              added in that order -- the same order, hence the same bits, on every run.  Buckets longer than
+//              kMaxSorted tokens are added in bucket order (still correct, order not fixed).  Bound by writing
+//              dW where most rows have no token (193 us for 128256 x 4096 and 8192 uniform tokens, 215 us when
+//              they are Zipf-distributed; 5.4 TB/s), by the load latency along a bucket where they are long.
 //
 // Indices outside [0, V) contribute nothing (forward: a zero row) and record kBadArgument in the
 // status word.
@@ -56,7 +56,6 @@ __global__ void embed_count_kernel(const int64_t* __restrict__ idx, int* __restr
 }
 
 constexpr int kScan = 1024;      // counts per CTA of the scan
-constexpr int kSumRows = 8;      // vocabulary rows per CTA of the sum
 
 __device__ __forceinline__ int block_sum_1024(int v, int* red) {      // every thread gets the sum
 #pragma unroll
@@ -78,13 +77,17 @@ __global__ void __launch_bounds__(kScan) embed_part_kernel(const int* __restrict
   if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
-// off[v] = cursor[v] = sum of cnt[0..v)
+// off[v] = cursor[v] = sum of cnt[0..v); without `part` the CTA adds up the counts in front of its own
 __global__ void __launch_bounds__(kScan) embed_scan_kernel(const int* __restrict__ cnt, const int* __restrict__ part,
                                                            int* __restrict__ off, int* __restrict__ cursor, int V) {
   __shared__ int red[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int before = 0;
-  for (int b = threadIdx.x; b < static_cast<int>(blockIdx.x); b += kScan) before += part[b];
+  if (part != nullptr) {
+    for (int b = threadIdx.x; b < static_cast<int>(blockIdx.x); b += kScan) before += part[b];
+  } else {
+    for (int b = 0; b < static_cast<int>(blockIdx.x); ++b) before += cnt[b * kScan + threadIdx.x];
+  }
   before = block_sum_1024(before, red);
   const int v = blockIdx.x * kScan + threadIdx.x;
   const int n = v < V ? cnt[v] : 0;
@@ -122,25 +125,29 @@ __device__ __forceinline__ void add_row(float (&acc)[8], const uint4& x) {
   }
 }
 
-// kSumRows vocabulary rows per CTA, a `stride` apart: ids follow frequency in most vocabularies, so that
-// neighbouring rows have long buckets together (eight consecutive rows: 566 us for 8192 Zipf-distributed
-// tokens, the first CTAs being the tail).  Thread c owns the 16-byte vector blockIdx.y * 256 + c.
-__global__ void __launch_bounds__(256) embed_sum_kernel(const uint4* __restrict__ dy, const int* __restrict__ cnt,
+// ROWS vocabulary rows per CTA, a `stride` apart: ids follow frequency in most vocabularies, so that
+// neighbouring rows have long buckets together.  The 256 threads own one vector each of 256 neighbouring ones.
+// CTAS per SM sets the registers: with 8 (32 registers) each token row of a bucket waits for the one before
+// it; with 4 (up to 64) eight are in flight, but rows without a token are cleared by half the threads.  Eight
+// rows per CTA left a vocabulary of a few thousand rows with too few CTAs (256 rows of 512, 65536 tokens:
+// 244 us; 60 now), and with more rows it was no faster than two.
+template <int ROWS, int CTAS>
+__global__ void __launch_bounds__(256, CTAS) embed_sum_kernel(const uint4* __restrict__ dy, const int* __restrict__ cnt,
                                                         const int* __restrict__ off, const int* __restrict__ bucket,
                                                         uint4* __restrict__ dw, int V, int stride, int vec_per_row) {
   __shared__ int raw[kMaxSorted];
   __shared__ int sorted[kMaxSorted];
-  const int c = blockIdx.y * 256 + threadIdx.x;
+  const int c = (blockIdx.z * gridDim.y + blockIdx.y) * 256 + threadIdx.x;
   const bool live = c < vec_per_row;
   for (int v0 = blockIdx.x; v0 < stride; v0 += gridDim.x) {
-    int counts[kSumRows];
+    int counts[ROWS];
 #pragma unroll
-    for (int i = 0; i < kSumRows; ++i) counts[i] = v0 + i * static_cast<int64_t>(stride) < V ? cnt[v0 + i * stride] : -1;
+    for (int i = 0; i < ROWS; ++i) counts[i] = v0 + i * static_cast<int64_t>(stride) < V ? cnt[v0 + i * stride] : -1;
 #pragma unroll
-    for (int i = 0; i < kSumRows; ++i)
+    for (int i = 0; i < ROWS; ++i)
       if (counts[i] == 0 && live) dw[static_cast<int64_t>(v0 + i * stride) * vec_per_row + c] = make_uint4(0, 0, 0, 0);
 #pragma unroll
-    for (int i = 0; i < kSumRows; ++i) {
+    for (int i = 0; i < ROWS; ++i) {
       const int n = counts[i];
       if (n <= 0) continue;                    // uniform over the CTA
       const int* b = bucket + off[v0 + i * stride];
@@ -221,16 +228,26 @@ extern "C" int hpb_embedding_bwd(const int64_t* idx, const void* dy, void* dw, i
     emb::embed_count_kernel<<<static_cast<unsigned>(want < sms * 8 ? want : sms * 8), 256, 0, s>>>(idx, cnt, T, V,
                                                                                                  status);
   }
-  emb::embed_part_kernel<<<scan_blocks, emb::kScan, 0, s>>>(cnt, part, V);
-  emb::embed_scan_kernel<<<scan_blocks, emb::kScan, 0, s>>>(cnt, part, off, cursor, V);
+  // up to 16384 rows a CTA of the scan adds up all counts in front of its own, which is shorter than a launch
+  // (1000 rows, 1000 tokens: 14.7 -> 12.6 us)
+  const bool direct = scan_blocks <= 16;
+  if (!direct) emb::embed_part_kernel<<<scan_blocks, emb::kScan, 0, s>>>(cnt, part, V);
+  emb::embed_scan_kernel<<<scan_blocks, emb::kScan, 0, s>>>(cnt, direct ? nullptr : part, off, cursor, V);
   if (T > 0) {
     const int64_t want = (T + 255) / 256;
     emb::embed_fill_kernel<<<static_cast<unsigned>(want < sms * 8 ? want : sms * 8), 256, 0, s>>>(idx, cursor, bucket,
                                                                                                 T, V);
   }
-  const int groups = (V + emb::kSumRows - 1) / emb::kSumRows;
-  const dim3 grid(groups < sms * 32 ? groups : sms * 32, (H / 8 + 255) / 256);
-  emb::embed_sum_kernel<<<grid, 256, 0, s>>>(reinterpret_cast<const uint4*>(dy), cnt, off, bucket,
-                                             reinterpret_cast<uint4*>(dw), V, groups, H / 8);
+  // Long buckets (more than 16 tokens per row on average): one row per CTA, and registers for eight token rows in
+  // flight.  Otherwise two rows per CTA and as many CTAs as fit.  Measured, one / two rows: 256 rows of 512, 65536
+  // tokens 60 / 93 us; 5000 rows of 512, 100000 tokens 43 / 47; 1024 rows of 4096, 8192 tokens 23.6 / 20.7; 32000 rows
+  // of 5120, 8192 tokens 137 / 86.
+  const bool dense = T > 16ll * V;
+  const int groups = dense ? V : (V + 1) / 2;
+  const int slices = (H / 8 + 255) / 256, planes = (slices + 65534) / 65535;
+  const dim3 grid(groups < sms * 32 ? groups : sms * 32, (slices + planes - 1) / planes, planes);
+  auto kern = dense ? emb::embed_sum_kernel<1, 4> : emb::embed_sum_kernel<2, 8>;
+  kern<<<grid, 256, 0, s>>>(reinterpret_cast<const uint4*>(dy), cnt, off, bucket, reinterpret_cast<uint4*>(dw), V, groups,
+                            H / 8);
   return static_cast<int>(cudaGetLastError());
 }
