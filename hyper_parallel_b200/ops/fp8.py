@@ -95,6 +95,15 @@ def dequantize(q, scale_act=None, scale_w=None) -> torch.Tensor:
     return (fp * scale_w[:, None, :, None]).view(nb * 128, K)[:N]
 
 
+def _wide_tiles(M: int, N: int, sms: int) -> bool:
+    """128x256 instead of 128x128 tiles.  A wide tile takes 1.2 to 1.35 times as long, so it wins as soon as it
+    saves the persistent grid a turn, and loses where it does not (K = 7168: 20000 x 64 61 against 51 us, 4096 x
+    1152 61 against 55; 4096 x 640 35 against 53, 20000 x 384 92 against 103, 20000 x 904 157 against 243).  Its
+    TMA stores need rows of whole 16-byte vectors."""
+    rows = -(-M // 128)
+    return N % 8 == 0 and -(-(rows * -(-N // 256)) // sms) < -(-(rows * -(-N // 128)) // sms)
+
+
 def gemm_fp8(aq, sa, bq, sb) -> torch.Tensor:
     """``C[M, N] = dequant(aq, sa) @ dequant(bq, sb).T`` in bf16, computed on the fp8 tensor cores."""
     M, K = aq.shape
@@ -103,14 +112,10 @@ def gemm_fp8(aq, sa, bq, sb) -> torch.Tensor:
         return (dequantize(aq, scale_act=sa) @ dequantize(bq, scale_w=sb).t()).to(torch.bfloat16)
     out = torch.empty((M, N), dtype=torch.bfloat16, device=aq.device)
     dev = aq.device
-    # A 128x256 tile takes about 1.5 times as long as a 128x128 one: the wide kernel wins as soon as the small
-    # tiles need a second wave (700 x 1536 x 7168, 72 small tiles: 37 against 32.5 us; 4096 x 576 x 7168, 160
-    # small tiles: 40 against 61 us).  Its TMA stores need rows of whole 16-byte vectors.
-    wide = N % 8 == 0 and -(-M // 128) * -(-N // 128) > native.sm_count(dev)
+    wide = _wide_tiles(M, N, native.sm_count(dev))
     fn = _lib().hpb_gemm_fp8_blockscale_wide if wide else _lib().hpb_gemm_fp8_blockscale
-    rc = fn(aq.data_ptr(), sa.data_ptr(), bq.data_ptr(), sb.data_ptr(), out.data_ptr(),
-                                        out.stride(0), M, N, K, native.status_word(dev).data_ptr(),
-                                        native.sm_count(dev), native.stream(dev))
+    rc = fn(aq.data_ptr(), sa.data_ptr(), bq.data_ptr(), sb.data_ptr(), out.data_ptr(), out.stride(0), M, N, K,
+            native.status_word(dev).data_ptr(), native.sm_count(dev), native.stream(dev))
     native.check(rc, "hpb_gemm_fp8_blockscale")
     return out
 
