@@ -256,9 +256,10 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
 constexpr float kE4M3Max = 448.f;
 
 // Both quantisers are bound by HBM (2 bytes read, 1 written per element).  A thread takes 16-byte vectors,
-// 16 neighbouring threads a 128-element tile row, and has its four or eight vectors in flight before the
-// first reduction.  Weights 36864 x 7168: 376 -> 121 us (6.6 TB/s), 7168 x 18432: 182 -> 64 us; activations
-// 4096 x 18432: 94 -> 50 us (4.6 TB/s), 4096 x 7168: 37 -> 20 us.
+// 16 neighbouring threads a 128-element tile row, and has its one, four or eight vectors in flight before the
+// first reduction.  Operands beyond L2: weights 36864 x 7168 376 -> 123 us (6.4 TB/s, two bytes read for each
+// one written; a copy runs at 6.46), 7168 x 18432 182 -> 64 us; activations 4096 x 18432 94 -> 49 us
+// (4.6 TB/s), 4096 x 7168 37 -> 21 us.
 
 // Eight bf16 values times `inv`, rounded to e4m3 (saturating).
 __device__ __forceinline__ uint2 to_e4m3(const uint4& u, float inv) {
@@ -284,38 +285,39 @@ __device__ __forceinline__ float abs_max(const uint4& u) {
   return m;
 }
 
-// x[M, K] bf16 -> q[M, K] e4m3, scales[K/128, M].  A CTA takes 32 rows x 256 columns: a warp 4 rows, half a
-// warp one tile; the scales go through shared memory so that the 32 of a column block leave as one line
-// (written one by one, 4 bytes every M * 4, they and the 8-byte loads held the kernel at 2.5 TB/s).
-constexpr int QA_ROWS = 32;
+// x[M, K] bf16 -> q[M, K] e4m3, scales[K/128, M].  A warp takes ROWS rows x 256 columns, half a warp one tile;
+// the scales of a CTA go through shared memory so that those of a column block leave as one segment (written one
+// by one, 4 bytes every M * 4, they and the 8-byte loads held the kernel at 2.5 TB/s).
+template <int ROWS>
 __global__ void __launch_bounds__(256)
 quant_act_1x128_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scales, int M,
                        int K) {
-  __shared__ float sc[2][QA_ROWS];
+  constexpr int CTA_ROWS = 8 * ROWS;
+  __shared__ float sc[2][CTA_ROWS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // (a grid's second dimension ends at 65535: 2^24 columns; the third goes on)
   const int kb0 = (blockIdx.z * gridDim.y + blockIdx.y) * 2, kblocks = K / 128;
   const int col = kb0 * 128 + lane * 8;
   const bool live = kb0 + (lane >> 4) < kblocks;
-  const int r0 = blockIdx.x * QA_ROWS + warp * 4;
-  uint4 v[4];
+  const int r0 = blockIdx.x * CTA_ROWS + warp * ROWS;
+  uint4 v[ROWS];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < ROWS; ++i)
     v[i] = live && r0 + i < M ? *reinterpret_cast<const uint4*>(x + static_cast<long long>(r0 + i) * K + col)
                               : make_uint4(0, 0, 0, 0);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < ROWS; ++i) {
     float amax = abs_max(v[i]);
 #pragma unroll
     for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
     const float scale = fmaxf(amax, 1e-10f) / kE4M3Max;
-    if ((lane & 15) == 0) sc[lane >> 4][warp * 4 + i] = scale;
+    if ((lane & 15) == 0) sc[lane >> 4][warp * ROWS + i] = scale;
     if (live && r0 + i < M)
       *reinterpret_cast<uint2*>(q + static_cast<long long>(r0 + i) * K + col) = to_e4m3(v[i], 1.f / scale);
   }
   __syncthreads();
-  if (warp < 2 && kb0 + warp < kblocks && blockIdx.x * QA_ROWS + lane < M)
-    scales[static_cast<long long>(kb0 + warp) * M + blockIdx.x * QA_ROWS + lane] = sc[warp][lane];
+  if (warp < 2 && lane < CTA_ROWS && kb0 + warp < kblocks && blockIdx.x * CTA_ROWS + lane < M)
+    scales[static_cast<long long>(kb0 + warp) * M + blockIdx.x * CTA_ROWS + lane] = sc[warp][lane];
 }
 
 // w[N, K] bf16 -> q[N, K] e4m3, scales[N/128, K/128]; one CTA per 128x128 block, thread = 8 rows x 16 bytes
@@ -427,9 +429,13 @@ extern "C" int hpb_quant_act_1x128(const void* x, void* q, float* scales, int M,
   // (cudaMalloc'ed or whole-row pointers are 16-byte aligned; K % 128 keeps every vector so)
   if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(q) & 7)) return -2;
   const int pairs = (K / 128 + 1) / 2, planes = (pairs + 65534) / 65535;
-  const dim3 grid((M + QA_ROWS - 1) / QA_ROWS, (pairs + planes - 1) / planes, planes);
-  quant_act_1x128_kernel<<<grid, 256, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<uint8_t*>(q),
-                                              scales, M, K);
+  // one row per warp instead of four up to two of the larger CTAs per SM: 128 x 512 1.75 against 2.35 us, 203 x 7168
+  // 2.3 / 2.8, 512 x 7168 3.4 / 3.6, 2000 x 7168 8.5 / 7.9, 4096 x 7168 17.6 / 15.5 (operands in L2)
+  const bool few = static_cast<long long>((M + 31) / 32) * pairs <= 2 * 148;
+  const int rows = few ? 8 : 32;
+  const dim3 grid((M + rows - 1) / rows, (pairs + planes - 1) / planes, planes);
+  auto kern = few ? quant_act_1x128_kernel<1> : quant_act_1x128_kernel<4>;
+  kern<<<grid, 256, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<uint8_t*>(q), scales, M, K);
   return static_cast<int>(cudaGetLastError());
 }
 

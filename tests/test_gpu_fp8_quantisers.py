@@ -1,5 +1,5 @@
 """The fp8 quantisers: the scales and bytes of the same steps on the CPU at row / column remainders
-(32 rows x 256 columns per CTA for activations, 128 x 128 for weights), on unaligned and strided input."""
+(8 or 32 rows x 256 columns per CTA for activations, 128 x 128 for weights), on unaligned and strided input."""
 import pytest
 import torch
 
@@ -23,7 +23,8 @@ def _same(got, want):
     assert torch.equal(got[0].cpu().view(torch.uint8), want[0].view(torch.uint8))
 
 
-@pytest.mark.parametrize("M,K", [(1, 128), (31, 384), (32, 256), (33, 128), (129, 640), (200, 7168)])
+@pytest.mark.parametrize("M,K", [(1, 128), (31, 384), (32, 256), (33, 128), (129, 640), (200, 7168),
+                                 (9, 256), (4099, 1408)])
 @pytest.mark.parametrize("form", ["plain", "strided", "offset", "special"])
 def test_quantisers(M, K, form):
     gen = torch.Generator(device="cuda").manual_seed(M + K)
