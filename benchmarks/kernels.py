@@ -62,12 +62,7 @@ def main():
     ap.add_argument("--small", action="store_true")
     ap.add_argument("--bwd-group", type=int, default=None,
                     help="attention backward: (batch, head) pairs scheduled together (0 = all, key-tile major)")
-    ap.add_argument("--mla-probe", type=int, default=0,
-                    help="timing probe of the MLA backward (wrong results): 1 = no dQ reduce, 2 = no exponentials, "
-                         "4 / 8 / 16 = without the dQ / dK, dV / score products")
     args = ap.parse_args()
-    if args.mla_probe:
-        native.lib().hpb_mla_attn_set_probe(args.mla_probe)
     if args.bwd_group is not None:
         native.lib().hpb_flash_attn_set_head_group(args.bwd_group)
         native.lib().hpb_mla_attn_set_head_group(args.bwd_group)

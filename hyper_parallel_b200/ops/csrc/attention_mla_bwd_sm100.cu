@@ -72,13 +72,10 @@ struct BwdParams {
   float scale, scale_log2;
   int causal;
   int head_group;        // (batch, head) pairs scheduled together
-  int probe;             // timing probes (results are wrong): 1 = no dQ staging / reduce, 2 = no exponentials,
-                         // 4 / 8 / 16 = the dQ^T / dK, dV / S^T, dP^T products are not issued
   const float* stats;    // [2][B, H, S]: lse * log2(e), rowsum(dO o O)
   __nv_bfloat16* dKV;    // [B, S, H, 256]: dK nope | dV
   __nv_bfloat16* dKR;    // [B, S, H, 64]: dK of the rotary columns, per head
   int* status;
-  long long* prof;       // optional [16]: cycles that one softmax thread of CTA 0 spent per phase, summed over its walk
 };
 
 __global__ void __launch_bounds__(BWD_THREADS, 1)
@@ -260,7 +257,6 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       auto issue_st = [&](int it) {
         if (!issuer) return;
         const uint64_t qa = desc_at(qk_desc, (it % RING) * Q_BYTES);
-        if (!(p.probe & 16))
 #pragma unroll
         for (int kb = 0; kb < 3; ++kb)
 #pragma unroll
@@ -273,7 +269,6 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       auto issue_dpt = [&](int it) {
         if (!issuer) return;
         const uint64_t doa = desc_at(dok_desc, (it % RING) * DO_BYTES);
-        if (!(p.probe & 16))
 #pragma unroll
         for (int kb = 0; kb < 2; ++kb)
 #pragma unroll
@@ -301,21 +296,10 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
           issue_st(1);
         }
       }
-      const bool prof = p.prof != nullptr && blockIdx.x == 0 && issuer;
-      long long acc[5] = {0, 0, 0, 0, 0};
-      long long tp = prof ? clock64() : 0;
-      auto tick = [&](int i) {
-        if (prof) {
-          const long long t = clock64();
-          acc[i] += t - tp;
-          tp = t;
-        }
-      };
       for (int it = 0; it < n_it && ok; ++it) {
         const int b = it & 1;
         ok = wait_on(&ds_full[b], (it >> 1) & 1, kTimeoutTmemFull);
         if (!ok) break;
-        tick(0);
         tc_fence_after();
         const uint64_t qa = desc_at(qm_desc, (it % RING) * Q_BYTES);
         const uint64_t doa = desc_at(dom_desc, (it % RING) * DO_BYTES);
@@ -324,12 +308,13 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         const uint32_t first = it ? 1u : 0u;
         // dV += P^T dO (contraction over the 64 query rows: 4 steps of 16).  P^T lies in the dP^T
         // buffer: query rows 0..31 in columns 0..15, 32..63 in columns 32..47 (8 columns per step)
-        if (issuer && !(p.probe & 8))
+        if (issuer) {
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-          umma_f16_ts(tmem_base + COL_DV, tmem_base + COL_DPT + (kk >> 1) * 32 + (kk & 1) * 8, desc_at(doa, kk * 2048),
-                      idesc_dv, kk ? 1u : first);
-        if (issuer) umma_commit(&do_empty[it % RING]);
+          for (int kk = 0; kk < 4; ++kk)
+            umma_f16_ts(tmem_base + COL_DV, tmem_base + COL_DPT + (kk >> 1) * 32 + (kk & 1) * 8,
+                        desc_at(doa, kk * 2048), idesc_dv, kk ? 1u : first);
+          umma_commit(&do_empty[it % RING]);
+        }
         // dP^T of the next step: its softmax is waiting for nothing else (executes behind dV, which
         // reads the buffer it overwrites)
         if (it + 1 < n_it) {
@@ -339,12 +324,12 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
           issue_dpt(it + 1);
         }
         // dK += dS^T Q; frees the Q slot, so that the load of step it + 2 starts early
-        if (issuer && !(p.probe & 8))
+        if (issuer) {
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-          umma_f16(tmem_base + COL_DK, desc_at(dsa, kk * 32), desc_at(qa, kk * 2048), idesc_dk, kk ? 1u : first);
-        if (issuer) umma_commit(&q_empty[it % RING]);
-        tick(1);
+          for (int kk = 0; kk < 4; ++kk)
+            umma_f16(tmem_base + COL_DK, desc_at(dsa, kk * 32), desc_at(qa, kk * 2048), idesc_dk, kk ? 1u : first);
+          umma_commit(&q_empty[it % RING]);
+        }
         // dQ^T = K^T dS^T (contraction over the 128 key rows: 8 steps of 16).  The rotary unit of K and a
         // neighbour (the unit in front of it in even steps, behind it -- V -- in odd ones, whose rows nobody
         // reads) go into the S^T buffer, free once the scores of step it + 1 are in registers (the three
@@ -354,13 +339,13 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
           if (!ok) break;
           tc_fence_after();
         }
-        tick(2);
-        if (issuer && !(p.probe & 4))
+        if (issuer) {
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          umma_f16(tmem_base + COL_ST, desc_at(kt_desc, (1 + b) * UNIT_BYTES + kk * 2048), desc_at(dsm, kk * 2048),
-                   idesc_dq, kk ? 1u : 0u);
-        if (issuer) umma_commit(dq_hi_full);
+          for (int kk = 0; kk < 8; ++kk)
+            umma_f16(tmem_base + COL_ST, desc_at(kt_desc, (1 + b) * UNIT_BYTES + kk * 2048), desc_at(dsm, kk * 2048),
+                     idesc_dq, kk ? 1u : 0u);
+          umma_commit(dq_hi_full);
+        }
         // head elements 0..127 (units 0, 1 of K) go into the dQ^T buffer, free once the tile of the
         // step before was read; this product runs while the upper tile is read out
         if (it > 0) {
@@ -368,12 +353,12 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
           if (!ok) break;
           tc_fence_after();
         }
-        if (issuer && !(p.probe & 4))
+        if (issuer) {
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          umma_f16(tmem_base + COL_DQ, desc_at(kt_desc, kk * 2048), desc_at(dsm, kk * 2048), idesc_dq, kk ? 1u : 0u);
-        if (issuer) umma_commit(dq_lo_full);
-        tick(3);
+          for (int kk = 0; kk < 8; ++kk)
+            umma_f16(tmem_base + COL_DQ, desc_at(kt_desc, kk * 2048), desc_at(dsm, kk * 2048), idesc_dq, kk ? 1u : 0u);
+          umma_commit(dq_lo_full);
+        }
         // The upper tile must have left the S^T buffer before anything else is written there: S^T of
         // step it + 2, or -- in the last two steps, where no score tile follows -- the upper tile of
         // the next step (this wait also keeps the phase of dq_hi_full at most one ahead of its readers)
@@ -387,10 +372,7 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
             issue_st(it + 2);
           }
         }
-        tick(4);
       }
-      if (prof)
-        for (int i = 0; i < 5; ++i) p.prof[10 + i] = acc[i];
       if (ok && issuer) umma_commit(acc_full);
       if (!ok && issuer) {
         umma_commit(drain_bar);
@@ -410,16 +392,6 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       const bool row_live = kv_row < p.S;
       const int sw = row & 7;
       const int c = wg;                       // this group's 32 query columns
-      const bool prof = p.prof != nullptr && blockIdx.x == 0 && threadIdx.x == 64;
-      long long acc[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-      long long tp = prof ? clock64() : 0;
-      auto tick = [&](int i) {
-        if (prof) {
-          const long long t = clock64();
-          acc[i] += t - tp;
-          tp = t;
-        }
-      };
       for (int it = 0; it < n_it && ok; ++it) {
         const int b = it & 1;
         // One wait for the scores, the row statistics and dS^T buffer b: S^T(it) was issued behind the barrier
@@ -427,7 +399,6 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         const float* stat = sStat + (it % RING) * 2 * BQ;
         ok = mbar_wait_bounded(st_full, it & 1, abort_flag, p.status, kTimeoutTmemFull, blockIdx.x);
         if (!ok) break;
-        tick(2);
         tc_fence_after();
         uint32_t rs[32];
         tmem_ld_32x32b_x32(tmem_base + COL_ST + c * 32 + lane_off, rs);
@@ -436,7 +407,6 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(st_consumed);
-        tick(3);
         const int q0 = (i_start + it) * BQ;
         // visible iff key <= query:  column c >= kv_row - q0
         const int cmin = p.causal ? kv_row - q0 : 0;
@@ -452,10 +422,8 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
             const float2 ls = *reinterpret_cast<const float2*>(stat + c * 32 + 2 * i2);
             float2 e = fma2(make_float2(__uint_as_float(rs[2 * i2]), __uint_as_float(rs[2 * i2 + 1])), sc2,
                             make_float2(-ls.x, -ls.y));
-            if (!(p.probe & 2)) {
-              e.x = fast_exp2(e.x);
-              e.y = fast_exp2(e.y);
-            }
+            e.x = fast_exp2(e.x);
+            e.y = fast_exp2(e.y);
             if (masked) {
               const int col = c * 32 + 2 * i2;
               if (!row_live || col < cmin) e.x = 0.f;
@@ -466,10 +434,8 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
             pk[i2] = *reinterpret_cast<const uint32_t*>(&eb);
           }
         }
-        tick(4);
         ok = mbar_wait_bounded(dpt_full, it & 1, abort_flag, p.status, kTimeoutTmemFull, blockIdx.x);
         if (!ok) break;
-        tick(5);
         tc_fence_after();
         {
           uint32_t rp[32], dk[16];
@@ -477,7 +443,6 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
           tmem_ld_wait();
           // P^T over the first 16 of the 32 columns just read (this thread's own)
           tmem_st_32x32b_x16(tmem_base + COL_DPT + c * 32 + lane_off, pk);
-          tick(6);
 #pragma unroll
           for (int i2 = 0; i2 < 16; ++i2) {
             const float2 dl = *reinterpret_cast<const float2*>(stat + BQ + c * 32 + 2 * i2);
@@ -493,17 +458,11 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
                 make_uint4(dk[4 * q4], dk[4 * q4 + 1], dk[4 * q4 + 2], dk[4 * q4 + 3]);
           }
         }
-        tick(7);
         tmem_st_wait();
         fence_proxy_async();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&ds_full[b]);
-        tick(8);
-      }
-      if (prof) {
-        for (int i = 0; i < 9; ++i) p.prof[i] = acc[i];
-        p.prof[9] = n_it;
       }
     } else {
       // ------------------------------------------------------ dQ reduction --
@@ -512,7 +471,6 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       // the fp32 dQ in global memory.  The upper product leaves the head elements 128..191 in lanes 64..127
       // in even steps and in lanes 0..63 in odd ones: two warps at a time pass a second tile through their
       // staging memory.
-      const bool staged = !(p.probe & 1);
       uint8_t* tile = sStage + quarter * STAGE_TILE;
       float* stage = reinterpret_cast<float*>(tile) + lane;
       for (int it = 0; it < n_it && ok; ++it) {
@@ -533,15 +491,13 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
             tma_store_wait_read<0>();                  // the tile of the step before has left the staging memory
           }
           __syncwarp();
-          if (staged) {
 #pragma unroll
-            for (int i = 0; i < 64; ++i) stage[i * 32] = __uint_as_float(r[i]) * p.scale;
-            fence_proxy_async();
-            __syncwarp();
-            if (lane == 0) {
-              tma_reduce_add_3d(&tmap_dq, tile, head * DQK + 128 + (quarter & 1) * 32, q0, batch);
-              tma_store_commit();
-            }
+          for (int i = 0; i < 64; ++i) stage[i * 32] = __uint_as_float(r[i]) * p.scale;
+          fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) {
+            tma_reduce_add_3d(&tmap_dq, tile, head * DQK + 128 + (quarter & 1) * 32, q0, batch);
+            tma_store_commit();
           }
         }
         ok = mbar_wait_bounded(dq_lo_full, it & 1, abort_flag, p.status, kTimeoutTmemFull, blockIdx.x);
@@ -557,15 +513,13 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
           tma_store_wait_read<0>();
         }
         __syncwarp();
-        if (staged) {
 #pragma unroll
-          for (int i = 0; i < 64; ++i) stage[i * 32] = __uint_as_float(r[i]) * p.scale;
-          fence_proxy_async();
-          __syncwarp();
-          if (lane == 0) {
-            tma_reduce_add_3d(&tmap_dq, tile, head * DQK + quarter * 32, q0, batch);
-            tma_store_commit();
-          }
+        for (int i = 0; i < 64; ++i) stage[i * 32] = __uint_as_float(r[i]) * p.scale;
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) {
+          tma_reduce_add_3d(&tmap_dq, tile, head * DQK + quarter * 32, q0, batch);
+          tma_store_commit();
         }
       }
       if (lane == 0) tma_store_wait<0>();
@@ -641,12 +595,6 @@ using namespace hpb;
 // Backward schedule: (batch, head) pairs per group; <= 0 = all pairs in one group (key-tile major).
 static int g_mla_bwd_head_group = 16;
 extern "C" void hpb_mla_attn_set_head_group(int pairs) { g_mla_bwd_head_group = pairs; }
-// Timing probes for the benchmarks (the gradients are wrong while one is set): see BwdParams::probe.
-static long long* g_mla_bwd_prof = nullptr;
-// Device buffer of 16 int64 that receives the phase timings of one softmax thread (nullptr = off).
-extern "C" void hpb_mla_attn_set_prof(long long* buf) { g_mla_bwd_prof = buf; }
-static int g_mla_bwd_probe = 0;
-extern "C" void hpb_mla_attn_set_probe(int mask) { g_mla_bwd_probe = mask; }
 
 // Backward.  q [B, S, H, 192], kv [B, S, H, 256] (k_nope | v), kr [B, S, 64], O / dO [B, S, H, 128] bf16
 // with the innermost dimension contiguous and row (token) / batch strides in elements; lse from the
@@ -712,8 +660,6 @@ extern "C" int hpb_mla_attn_bwd(const void* q, long long q_batch_stride, long lo
   p.scale_log2 = softmax_scale * 1.4426950408889634f;
   p.causal = causal;
   p.head_group = g_mla_bwd_head_group > 0 ? g_mla_bwd_head_group : (1 << 30);
-  p.probe = g_mla_bwd_probe;
-  p.prof = g_mla_bwd_prof;
   p.stats = stats;
   p.dKV = reinterpret_cast<__nv_bfloat16*>(dKV);
   p.dKR = reinterpret_cast<__nv_bfloat16*>(dkr_heads);

@@ -3,7 +3,7 @@ import re
 
 import pytest
 
-from hyper_parallel_b200.ops import build
+from hyper_parallel_b200.ops import build, native
 
 
 def _entries():
@@ -19,3 +19,11 @@ def test_gemm_accumulators_stay_in_registers():
     gemms = [(name, int(frame)) for name, frame in _entries() if re.search(r"gemm\w*_kernel", name)]
     assert len(gemms) > 40
     assert not [name for name, frame in gemms if frame]
+
+
+@pytest.mark.parametrize("name", ["hpb_mla_attn_set_probe", "hpb_mla_attn_set_prof"])
+def test_no_switch_that_skips_work(name):
+    """A library call must not be able to leave parts of a kernel out."""
+    if not native.available():
+        pytest.skip("the library has not been built")
+    assert not hasattr(native.lib(), name)
