@@ -6,7 +6,7 @@ the fly -- package name, ``"npu"`` device strings and ``.npu()`` calls, the HCCL
 ``torch_npu`` import -- and runs one of its functions, or all of them, on ``gloo`` ranks:
 
     python -m hyper_parallel_b200.utils.reference_compat --root <checkout of the reference> \\
-        tests/torch/shard/submesh.py [test_function] [--world 8]
+        tests/torch/shard/submesh.py [test_function] [--world 8] [--work-dir <folder for what the tests save>]
 
 Helper modules the tests import (``tests.torch.utils``, ``tests.torch.common_net``,
 ``tests.torch.shard.utils``, ``tests.torch.hsdp.hsdp_test_common``) are rewritten the same way, with
@@ -166,8 +166,14 @@ def main(argv=None) -> int:
     ap.add_argument("function", nargs="?", help="one test function (default: every test_* of the file)")
     ap.add_argument("--world", type=int, default=8)
     ap.add_argument("--timeout", type=float, default=600.0)
+    ap.add_argument("--work-dir", help="folder to run in (created): tests that save write relative paths, and some load "
+                                       "what another one saved; default: the current folder")
     ns = ap.parse_args(argv)
+    ns.root = os.path.abspath(ns.root)
     failed = 0
+    if ns.work_dir:
+        os.makedirs(ns.work_dir, exist_ok=True)
+        os.chdir(ns.work_dir)
     with tempfile.TemporaryDirectory(prefix="hpb_compat_") as out_root:
         path = prepare(ns.root, ns.file, out_root)
         functions = [ns.function] if ns.function else list_test_functions(os.path.join(ns.root, ns.file))

@@ -1,6 +1,9 @@
 """custom_shard, parallelize_value_and_grad, custom distributed-op registration through the
 environment, DeviceMesh.from_group / flatten, and tied parameters across pipeline stages."""
 import os
+import subprocess
+import sys
+from pathlib import Path
 
 import pytest
 import torch
@@ -209,6 +212,24 @@ def test_reference_compat_runner_rewrites_and_runs_a_reference_style_test(tmp_pa
     assert ok and tb is None
     ok, tb = rc.run_function(str(out), path, "test_that_fails", 2, timeout=120.0)
     assert not ok and "as intended" in tb
+
+
+def test_reference_compat_runner_keeps_what_tests_save_out_of_the_current_folder(tmp_path):
+    root = tmp_path / "checkout"
+    (root / "tests" / "torch" / "demo").mkdir(parents=True)
+    (root / "tests" / "torch" / "demo" / "save_case.py").write_text(
+        "from pathlib import Path\n\n\n"
+        "def test_save():\n"
+        "    Path('saved_here').mkdir(exist_ok=True)\n"
+        "    assert not Path('checkout').exists()\n")
+    cur = tmp_path / "cur"
+    cur.mkdir()
+    r = subprocess.run([sys.executable, "-m", "hyper_parallel_b200.utils.reference_compat", "--root", "../checkout",
+                        "tests/torch/demo/save_case.py", "--world", "2", "--work-dir", "../work"], cwd=cur,
+                       env=dict(os.environ, PYTHONPATH=str(Path(__file__).resolve().parents[1])), capture_output=True,
+                       text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+    assert (tmp_path / "work" / "saved_here").is_dir() and not list(cur.iterdir())
 
 
 def test_platform_facade_offers_the_reference_method_names():
