@@ -134,7 +134,8 @@ __device__ __forceinline__ void add_row(float (&acc)[8], const uint4& x) {
 template <int ROWS, int CTAS>
 __global__ void __launch_bounds__(256, CTAS) embed_sum_kernel(const uint4* __restrict__ dy, const int* __restrict__ cnt,
                                                         const int* __restrict__ off, const int* __restrict__ bucket,
-                                                        uint4* __restrict__ dw, int V, int stride, int vec_per_row) {
+                                                        uint4* __restrict__ dw, int V, int stride, int vec_per_row,
+                                                        int64_t T, int* status) {
   __shared__ int raw[kMaxSorted];
   __shared__ int sorted[kMaxSorted];
   const int c = (blockIdx.z * gridDim.y + blockIdx.y) * 256 + threadIdx.x;
@@ -152,6 +153,10 @@ __global__ void __launch_bounds__(256, CTAS) embed_sum_kernel(const uint4* __res
       if (n <= 0) continue;                    // uniform over the CTA
       const int* b = bucket + off[v0 + i * stride];
       const int* order = b;
+      bool ok = true;                          // (nothing in the normal build)
+      for (int k = 0; k < n; ++k)
+        ok = ok && HPB_BOUNDS_OK(b[k] >= 0 && b[k] < T, status, 0x900000 | (blockIdx.x & 0xffff));
+      if (!ok) continue;                       // uniform over the CTA
       if (n > 1 && n <= kMaxSorted) {
         __syncthreads();                       // the previous row's readers are done with the arrays
         for (int k = threadIdx.x; k < n; k += 256) raw[k] = b[k];
@@ -204,12 +209,7 @@ extern "C" int hpb_embedding_fwd(const int64_t* idx, const void* w, void* out, i
   return static_cast<int>(cudaGetLastError());
 }
 
-// Number of int32 words of scratch that hpb_embedding_bwd needs.
-extern "C" int64_t hpb_embedding_bwd_scratch_words(int64_t T, int V) {
-  return 3ll * V + T + (V + hpb::emb::kScan - 1) / hpb::emb::kScan;
-}
-
-// dw[V, H] = scatter-add of dy[T, H] by idx (every row written); scratch: hpb_embedding_bwd_scratch_words ints.
+// dw[V, H] = scatter-add of dy[T, H] by idx (every row written); scratch: 3 V + T + ceil(V / 1024) ints.
 extern "C" int hpb_embedding_bwd(const int64_t* idx, const void* dy, void* dw, int* scratch, int64_t T, int V, int H,
                                  int* status, int num_sms, cudaStream_t s) {
   if (H <= 0 || H % 8 || V <= 0 || T < 0 || T > 0x7fffffff) return -2;
@@ -248,6 +248,6 @@ extern "C" int hpb_embedding_bwd(const int64_t* idx, const void* dy, void* dw, i
   const dim3 grid(groups < sms * 32 ? groups : sms * 32, (slices + planes - 1) / planes, planes);
   auto kern = dense ? emb::embed_sum_kernel<1, 4> : emb::embed_sum_kernel<2, 8>;
   kern<<<grid, 256, 0, s>>>(reinterpret_cast<const uint4*>(dy), cnt, off, bucket, reinterpret_cast<uint4*>(dw), V, groups,
-                            H / 8);
+                            H / 8, T, status);
   return static_cast<int>(cudaGetLastError());
 }

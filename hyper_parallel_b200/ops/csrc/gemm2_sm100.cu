@@ -63,7 +63,9 @@ __device__ __forceinline__ Tile tile_at(int t, int num_m, int num_n, const Param
     ti.num_k = (r1 - r0 + BLOCK_K - 1) / BLOCK_K;
   } else {
     tile_coords(t, num_m, num_n, ti.m_blk, ti.n_blk);
-    ti.group = min(g.block_group[ti.m_blk], g.num_groups - 1);
+    ti.group = g.block_group[ti.m_blk];
+    if (!HPB_BOUNDS_OK(ti.group < g.num_groups, p.status, 0x700000 | ti.m_blk)) ti.group = -1;   // debug build: skip
+    ti.group = min(ti.group, g.num_groups - 1);
     ti.k_row0 = 0;
     ti.num_k = ti.group < 0 ? 0 : (p.K + BLOCK_K - 1) / BLOCK_K;
   }

@@ -110,7 +110,8 @@ __global__ void tables_kernel(const int* __restrict__ starts, const int* __restr
 
 __global__ void __launch_bounds__(CHUNK) place_kernel(const int64_t* __restrict__ idx, const int* __restrict__ hist,
                                                       const int* __restrict__ starts, int* __restrict__ pos,
-                                                      int* __restrict__ row_pair, int64_t pairs, int E) {
+                                                      int* __restrict__ row_pair, int64_t pairs, int E, int64_t rows,
+                                                      int* status) {
   __shared__ int ids[CHUNK];
   const int64_t i = blockIdx.x * static_cast<int64_t>(CHUNK) + threadIdx.x;
   const int e = i < pairs ? static_cast<int>(idx[i]) : -1;
@@ -121,14 +122,16 @@ __global__ void __launch_bounds__(CHUNK) place_kernel(const int64_t* __restrict_
   for (int j = 0; j < threadIdx.x; ++j) rank += ids[j] == e;
   const int r = starts[e] + hist[static_cast<int64_t>(e) * gridDim.x + blockIdx.x] + rank;
   pos[i] = r;
-  row_pair[r] = static_cast<int>(i);
+  if (HPB_BOUNDS_OK(r >= 0 && r < rows, status, 0x800000 | e)) row_pair[r] = static_cast<int>(i);
 }
 
 // xp[row] = x[pair / k], zeros in padding rows; one row per blockIdx.x
 __global__ void __launch_bounds__(256) gather_kernel(const uint4* __restrict__ x, const int* __restrict__ row_pair,
-                                                     uint4* __restrict__ xp, int k, int vecs) {
+                                                     uint4* __restrict__ xp, int k, int vecs, int64_t pairs,
+                                                     int* status) {
   const int64_t row = blockIdx.x;
-  const int pair = row_pair[row];
+  int pair = row_pair[row];
+  if (!HPB_BOUNDS_OK(pair < pairs, status, 0x810000 | (blockIdx.x & 0xffff))) pair = -1;
   uint4* dst = xp + row * vecs;
   if (pair < 0) {
     for (int c = threadIdx.x; c < vecs; c += 256) dst[c] = make_uint4(0, 0, 0, 0);
@@ -150,9 +153,11 @@ __global__ void __launch_bounds__(256) gather_kernel(const uint4* __restrict__ x
 // Four rows are in flight per thread.
 __global__ void __launch_bounds__(256) combine_kernel(const uint4* __restrict__ yp, const int* __restrict__ pos,
                                                       const float* __restrict__ w, uint4* __restrict__ out, int k,
-                                                      int vecs) {
+                                                      int vecs, int64_t rows, int* status) {
   const int64_t t = blockIdx.x;
   const int* p = pos + t * k;
+  for (int j = 0; j < k; ++j)      // (nothing in the normal build)
+    if (!HPB_BOUNDS_OK(p[j] >= 0 && p[j] < rows, status, 0x820000 | (blockIdx.x & 0xffff))) return;
   for (int c = threadIdx.x; c < vecs; c += 256) {
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     for (int j0 = 0; j0 < k; j0 += 4) {
@@ -180,10 +185,11 @@ __global__ void __launch_bounds__(256) combine_kernel(const uint4* __restrict__ 
 __global__ void __launch_bounds__(256) combine_bwd_kernel(const uint4* __restrict__ dout, const int* __restrict__ row_pair,
                                                           const float* __restrict__ w, const uint4* __restrict__ yp,
                                                           uint4* __restrict__ dyp, float* __restrict__ dw, int k,
-                                                          int vecs) {
+                                                          int vecs, int64_t pairs, int* status) {
   __shared__ float red[8];
   const int64_t row = blockIdx.x;
-  const int pair = row_pair[row];
+  int pair = row_pair[row];
+  if (!HPB_BOUNDS_OK(pair < pairs, status, 0x830000 | (blockIdx.x & 0xffff))) pair = -1;
   uint4* dst = dyp + row * vecs;
   if (pair < 0) {
     for (int c = threadIdx.x; c < vecs; c += 256) dst[c] = make_uint4(0, 0, 0, 0);
@@ -236,11 +242,8 @@ __global__ void __launch_bounds__(256) combine_bwd_kernel(const uint4* __restric
 
 using namespace hpb::moel;
 
-// Number of int32 words of `hist` for hpb_moe_plan.
-extern "C" int64_t hpb_moe_plan_words(int64_t pairs, int E) { return (pairs + CHUNK - 1) / CHUNK * E; }
-
 // First half of the plan: counts / starts / ends [E]; counts[E] becomes non-zero when an expert id is out
-// of range.  E <= 8192.
+// of range.  E <= 8192; hist: E words for every 256 pairs.
 extern "C" int hpb_moe_count(const int64_t* idx, int* hist, int* counts, int* starts, int* ends, int64_t pairs, int E,
                              int pad, cudaStream_t s) {
   if (pairs <= 0 || pairs > 0x3fffffff || E <= 0 || E > 8192 || pad <= 0) return -2;
@@ -255,11 +258,12 @@ extern "C" int hpb_moe_count(const int64_t* idx, int* hist, int* counts, int* st
 
 // Second half (every id in range): block_group [rows / pad], row_pair [rows], pos [pairs].
 extern "C" int hpb_moe_place(const int64_t* idx, const int* hist, const int* starts, const int* ends, int* block_group,
-                             int* row_pair, int* pos, int64_t pairs, int E, int pad, cudaStream_t s) {
+                             int* row_pair, int* pos, int64_t pairs, int E, int pad, int64_t rows, int* status,
+                             cudaStream_t s) {
   if (pairs <= 0 || pairs > 0x3fffffff || E <= 0 || pad <= 0) return -2;
   tables_kernel<<<E, 128, 0, s>>>(starts, ends, E, pad, block_group, row_pair);
   place_kernel<<<static_cast<unsigned>((pairs + CHUNK - 1) / CHUNK), CHUNK, 0, s>>>(idx, hist, starts, pos, row_pair,
-                                                                                 pairs, E);
+                                                                                 pairs, E, rows, status);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -267,29 +271,31 @@ static bool aligned16(const void* a, const void* b, const void* c = nullptr) {
   return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15) == 0;
 }
 
-extern "C" int hpb_moe_gather(const void* x, const int* row_pair, void* xp, int64_t rows, int k, int H, cudaStream_t s) {
+// (rows / pairs and status below: what the index checks of the debug build compare with and report to)
+extern "C" int hpb_moe_gather(const void* x, const int* row_pair, void* xp, int64_t rows, int k, int H, int64_t pairs,
+                              int* status, cudaStream_t s) {
   if (H % 8 || k <= 0 || rows > 0x7fffffff || !aligned16(x, xp)) return -2;
   if (rows <= 0) return 0;
   gather_kernel<<<static_cast<unsigned>(rows), 256, 0, s>>>(reinterpret_cast<const uint4*>(x), row_pair,
-                                                            reinterpret_cast<uint4*>(xp), k, H / 8);
+                                                            reinterpret_cast<uint4*>(xp), k, H / 8, pairs, status);
   return static_cast<int>(cudaGetLastError());
 }
 
 extern "C" int hpb_moe_combine(const void* yp, const int* pos, const float* w, void* out, int64_t T, int k, int H,
-                               cudaStream_t s) {
+                               int64_t rows, int* status, cudaStream_t s) {
   if (H % 8 || k <= 0 || T > 0x7fffffff || !aligned16(yp, out)) return -2;
   if (T <= 0) return 0;
   combine_kernel<<<static_cast<unsigned>(T), 256, 0, s>>>(reinterpret_cast<const uint4*>(yp), pos, w,
-                                                          reinterpret_cast<uint4*>(out), k, H / 8);
+                                                          reinterpret_cast<uint4*>(out), k, H / 8, rows, status);
   return static_cast<int>(cudaGetLastError());
 }
 
 extern "C" int hpb_moe_combine_bwd(const void* dout, const int* row_pair, const float* w, const void* yp, void* dyp,
-                                   float* dw, int64_t rows, int k, int H, cudaStream_t s) {
+                                   float* dw, int64_t rows, int k, int H, int64_t pairs, int* status, cudaStream_t s) {
   if (H % 8 || k <= 0 || rows > 0x7fffffff || !aligned16(dout, dyp, yp)) return -2;
   if (rows <= 0) return 0;
   combine_bwd_kernel<<<static_cast<unsigned>(rows), 256, 0, s>>>(
       reinterpret_cast<const uint4*>(dout), row_pair, w, reinterpret_cast<const uint4*>(yp),
-      reinterpret_cast<uint4*>(dyp), dw, k, H / 8);
+      reinterpret_cast<uint4*>(dyp), dw, k, H / 8, pairs, status);
   return static_cast<int>(cudaGetLastError());
 }

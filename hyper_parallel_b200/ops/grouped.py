@@ -117,10 +117,10 @@ def _local_lib():
         lib.hpb_gemm2_bf16_grouped.argtypes = [vp, c64, c64, vp, ci, c64, c64, vp, c64, ci, ci, ci, ci, vp, vp, vp, ci,
                                                ci, vp, ci, vp]
         lib.hpb_moe_count.argtypes = [vp, vp, vp, vp, vp, c64, ci, ci, vp]
-        lib.hpb_moe_place.argtypes = [vp, vp, vp, vp, vp, vp, vp, c64, ci, ci, vp]
-        lib.hpb_moe_gather.argtypes = [vp, vp, vp, c64, ci, ci, vp]
-        lib.hpb_moe_combine.argtypes = [vp, vp, vp, vp, c64, ci, ci, vp]
-        lib.hpb_moe_combine_bwd.argtypes = [vp, vp, vp, vp, vp, vp, c64, ci, ci, vp]
+        lib.hpb_moe_place.argtypes = [vp, vp, vp, vp, vp, vp, vp, c64, ci, ci, c64, vp, vp]
+        lib.hpb_moe_gather.argtypes = [vp, vp, vp, c64, ci, ci, c64, vp, vp]
+        lib.hpb_moe_combine.argtypes = [vp, vp, vp, vp, c64, ci, ci, c64, vp, vp]
+        lib.hpb_moe_combine_bwd.argtypes = [vp, vp, vp, vp, vp, vp, c64, ci, ci, c64, vp, vp]
         lib._hpb_moe_local_bound = True
     return lib
 
@@ -185,7 +185,7 @@ class _Plan:
         self.slots = torch.empty(rows // pad + rows + pairs, dtype=torch.int32, device=dev)
         native.check(lib.hpb_moe_place(idx.data_ptr(), hist.data_ptr(), starts, starts + 4 * E, self.slots.data_ptr(),
                                        _row_pair(self.slots, self.dims), _pos(self.slots, self.dims), pairs, E, pad,
-                                       stream), "hpb_moe_place")
+                                       rows, native.status_word(dev).data_ptr(), stream), "hpb_moe_place")
 
 
 def _row_pair(slots, dims):
@@ -214,7 +214,7 @@ class _ExpertRows(torch.autograd.Function):
         _, F2, H = w_gate_up.shape
         xp = torch.empty((rows, H), dtype=x.dtype, device=dev)
         native.check(lib.hpb_moe_gather(x.data_ptr(), _row_pair(plan.slots, plan.dims), xp.data_ptr(), rows, k, H,
-                                        stream), "hpb_moe_gather")
+                                        T * k, native.status_word(dev).data_ptr(), stream), "hpb_moe_gather")
         gu = torch.empty((rows, F2), dtype=x.dtype, device=dev)
         _expert_rows(xp, w_gate_up, gu, plan.slots, pad, False)
         act = torch.empty((rows, F2 // 2), dtype=x.dtype, device=dev)
@@ -252,15 +252,17 @@ class _ExpertRows(torch.autograd.Function):
                 _expert_rows(dgu, w_gate_up, dxp, slots, pad, True)
                 dx = torch.empty((T, H), dtype=dt, device=dev)
                 native.check(lib.hpb_moe_combine(dxp.data_ptr(), _pos(slots, ctx.dims), None, dx.data_ptr(), T, k, H,
-                                                 stream), "hpb_moe_combine")
+                                                 rows, native.status_word(dev).data_ptr(), stream), "hpb_moe_combine")
         return dx, dw1, dw2, None
 
 
 def _combine_rows(yp, gate, slots, dims):
-    T, k, _, _, _ = dims
-    y = torch.empty((T, yp.shape[1]), dtype=yp.dtype, device=yp.device)
-    native.check(_local_lib().hpb_moe_combine(yp.data_ptr(), _pos(slots, dims), gate.data_ptr(), y.data_ptr(), T, k,
-                                              yp.shape[1], native.stream(yp.device)), "hpb_moe_combine")
+    T, k, _, rows, _ = dims
+    dev, H = yp.device, yp.shape[1]
+    y = torch.empty((T, H), dtype=yp.dtype, device=dev)
+    native.check(_local_lib().hpb_moe_combine(yp.data_ptr(), _pos(slots, dims), gate.data_ptr(), y.data_ptr(), T, k, H,
+                                              rows, native.status_word(dev).data_ptr(), native.stream(dev)),
+                 "hpb_moe_combine")
     return y
 
 
@@ -295,6 +297,7 @@ class _Combine(torch.autograd.Function):
         dgate = torch.empty((T, k), dtype=torch.float32, device=dy.device) if need_gate else None
         native.check(_local_lib().hpb_moe_combine_bwd(dy.data_ptr(), _row_pair(slots, ctx.dims), gate.data_ptr(),
                                                       native.ptr(yp), dyp.data_ptr(), native.ptr(dgate), rows, k, H,
+                                                      T * k, native.status_word(dy.device).data_ptr(),
                                                       native.stream(dy.device)), "hpb_moe_combine_bwd")
         return dyp, dgate, None
 
