@@ -97,8 +97,9 @@ __device__ __forceinline__ void store_row32_elements(T* dst, const uint32_t (&r)
     if (j < n) dst[j] = static_cast<T>(ACCUM ? __uint_as_float(r[j]) + old[j] : __uint_as_float(r[j]));
 }
 
-// Tensor map of C as [slices][rows][cols] for epilogue_tma (box: 32 rows x 128 bytes); false when the
-// pointer or the row stride is not a multiple of 16 bytes (the kernels then store element by element).
+// Tensor map of C as [slices][rows][cols] for epilogue_tma (box: 32 rows x 128 bytes); false when the pointer,
+// the row stride or the width is not a multiple of 16 bytes.  The kernels then take plain stores: of 16 bytes as
+// far as whole vectors go where the rows start on 16-byte boundaries, else element by element.
 bool make_tmap_c(CUtensorMap* map, void* c, bool f32, uint64_t cols, uint64_t rows, uint64_t slices, int64_t ldc);
 
 }  // namespace hpb

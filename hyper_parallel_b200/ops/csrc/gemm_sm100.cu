@@ -404,7 +404,8 @@ int make_tmap_2d(CUtensorMap* map, const void* ptr, CUtensorMapDataType dtype, i
 
 bool make_tmap_c(CUtensorMap* map, void* c, bool f32, uint64_t cols, uint64_t rows, uint64_t slices, int64_t ldc) {
   const uint64_t esize = f32 ? 4 : 2;
-  if ((reinterpret_cast<uintptr_t>(c) & 15) || (ldc * esize) % 16 || ldc < static_cast<int64_t>(cols)) return false;
+  // (a TMA store clips whole 16-byte vectors: columns that end inside one would be followed by zeros)
+  if (!rows_aligned16(c, ldc * esize) || (cols * esize) % 16 || ldc < static_cast<int64_t>(cols)) return false;
   EncodeTiledFn enc = get_encode_fn();
   if (enc == nullptr) return false;
   cuuint64_t dims[3] = {cols, rows, slices};

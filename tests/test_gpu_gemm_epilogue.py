@@ -41,6 +41,31 @@ def test_store_window(pair, dtype, M, N, K, front, extra):
 
 @pytest.mark.parametrize("pair", ["0", "1"])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("M,N", [(1, 1), (33, 41), (130, 67), (257, 1003)])
+@pytest.mark.parametrize("front", [0, 8])
+def test_columns_that_end_inside_a_vector(pair, dtype, M, N, front):
+    """TMA stores into rows of whole 16-byte vectors, clipped in the middle of one: the columns behind stay."""
+    gen = torch.Generator(device="cuda").manual_seed(M + N)
+    a = torch.randn(M, 72, device="cuda", generator=gen).to(torch.bfloat16)
+    b = torch.randn(N, 72, device="cuda", generator=gen).to(torch.bfloat16)
+    buf = torch.full((M + 2, front + (N + 7) // 8 * 8 + 8), 7.0, device="cuda", dtype=dtype)
+    out = buf[1:M + 1, front:front + N]
+    assert out.data_ptr() % 16 == 0 and out.stride(0) * out.element_size() % 16 == 0
+    Fn.set_gemm_pair_mode(pair)
+    try:
+        Fn.gemm(a, b, out=out)
+    finally:
+        Fn.set_gemm_pair_mode("auto")
+    native.check_status()
+    ref = a.double() @ b.double().t()
+    assert ((out.double() - ref).norm() / ref.norm()).item() < TOL[dtype]
+    rest = buf.clone()
+    rest[1:M + 1, front:front + N] = 7.0
+    assert (rest == 7.0).all()
+
+
+@pytest.mark.parametrize("pair", ["0", "1"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("front,extra", [(0, 0), (1, 7), (6, 2), (3, 0)])
 def test_accumulate_window(pair, dtype, front, extra):
     M, N, K = 257, 264, 72
