@@ -321,9 +321,10 @@ def test_flash_attention_backward(B, S, H, Hkv, causal):
     assert _rel_err(dq, rq) < 2e-2
 
 
-def test_fused_expert_ffn_single_rank_matches_reference_path():
-    """EP = 1: dispatch / combine kernels + grouped GEMMs against the index-select formulation."""
-    from hyper_parallel_b200.ops import moe
+def test_fused_expert_ffn_single_rank_matches_reference_path(monkeypatch):
+    """EP = 1: dispatch / combine kernels + grouped GEMMs against the layer in 64 bits and against the index-select
+    formulation (not the one-GPU kernels that ``expert_parallel_ffn`` would take here)."""
+    from hyper_parallel_b200.ops import grouped, moe
     from hyper_parallel_b200.parallel import ep_fused
     torch.manual_seed(9)
     T, H, Fh, E, k = 300, 256, 128, 8, 3
@@ -344,10 +345,22 @@ def test_fused_expert_ffn_single_rank_matches_reference_path():
         y.backward(dy)
         return [y] + [t.grad for t in (xa, wa, ga, da)]
 
-    got, ref = run(True), run(False)
+    def oracle():
+        xa, wa, ga, da = [t.double().requires_grad_() for t in (x, wts, wgu, wd)]
+        y = torch.zeros_like(xa)
+        for e in range(E):
+            tok, slot = (idx == e).nonzero(as_tuple=True)
+            g, u = (xa[tok] @ ga[e].t()).chunk(2, -1)
+            y = y.index_add(0, tok, (torch.nn.functional.silu(g) * u) @ da[e].t() * wa[tok, slot][:, None])
+        y.backward(dy.double())
+        return [y] + [t.grad for t in (xa, wa, ga, da)]
+
+    monkeypatch.setattr(grouped, "local_experts_usable", lambda *a: False)
+    got, general, exact = run(True), run(False), oracle()
     native.check_status()
-    for a, b, name in zip(got, ref, ["y", "dx", "dw_topk", "dw_gate_up", "dw_down"]):
+    for a, b, c, name in zip(got, general, exact, ["y", "dx", "dw_topk", "dw_gate_up", "dw_down"]):
         assert _rel_err(a, b) < 2e-2, name
+        assert ((a.double() - c).norm() / c.norm()).item() < 2e-2, name
 
 
 @pytest.mark.gpu

@@ -90,8 +90,10 @@ def test_expert_id_out_of_range_is_refused(bad):
     args = list(_inputs(9, 2, 4, 64, 16, "plain"))
     args[1] = args[1].clone()
     args[1][3, 1] = bad
-    with pytest.raises(Exception):
+    with pytest.raises(ValueError, match="expert ids must lie in"):
         moe.expert_parallel_ffn(*args[:3], args[3], args[4], 4)
+    good = _inputs(9, 2, 4, 64, 16, "plain")                   # nothing was launched on the bad ids
+    assert _err(_pass(moe.expert_parallel_ffn, *good)[0], _oracle(*good)[0]) < TOL
 
 
 def test_frozen_weights_and_inputs():
