@@ -12,11 +12,12 @@
 //   dV  += P^T dO           [kv 128 x 128]    accumulated over the whole walk
 //   dK  += dS^T Q           [kv 128 x 192]    accumulated over the whole walk
 //   dQ^T = K^T dS^T         [d 192 x q 64]    as two products of 128 rows: head elements 0..127 into
-//                                             a buffer of their own; elements 128..191 into the S^T
-//                                             buffer between two score tiles, in rows 64..127 (even
-//                                             steps) or 0..63 (odd steps), so that the four read-out
-//                                             warps share the work: 3 tiles per 2 steps each, not 2
-//                                             for two of them and 4 for the others
+//                                             a buffer of their own, 64..191 (of which rows 64..127 =
+//                                             elements 128..191 are read out) into the S^T buffer
+//                                             between two score tiles.  (Tried: the rotary rows in lanes
+//                                             64..127 and 0..63 in turn, so that the four read-out warps
+//                                             share the work: no faster, S = 4096, 128 heads 2627 against
+//                                             2629 us)
 //
 // Tensor memory (512 columns): S^T 64 | dP^T 64 | dQ^T 64 | dV 128 | dK 192.  The two accumulators
 // leave room for three 64-column buffers only, so nothing is double buffered; instead every buffer
@@ -330,10 +331,9 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
             umma_f16(tmem_base + COL_DK, desc_at(dsa, kk * 32), desc_at(qa, kk * 2048), idesc_dk, kk ? 1u : first);
           umma_commit(&q_empty[it % RING]);
         }
-        // dQ^T = K^T dS^T (contraction over the 128 key rows: 8 steps of 16).  The rotary unit of K and a
-        // neighbour (the unit in front of it in even steps, behind it -- V -- in odd ones, whose rows nobody
-        // reads) go into the S^T buffer, free once the scores of step it + 1 are in registers (the three
-        // products above have kept the tensor core busy meanwhile)
+        // dQ^T = K^T dS^T (contraction over the 128 key rows: 8 steps of 16).  Head elements 64..191
+        // (units 1, 2 of K) go into the S^T buffer, free once the scores of step it + 1 are in
+        // registers (the three products above have kept the tensor core busy meanwhile)
         if (it + 1 < n_it) {
           ok = wait_on(st_consumed, (it + 1) & 1, kTimeoutTmemEmpty);
           if (!ok) break;
@@ -342,8 +342,8 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         if (issuer) {
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk)
-            umma_f16(tmem_base + COL_ST, desc_at(kt_desc, (1 + b) * UNIT_BYTES + kk * 2048), desc_at(dsm, kk * 2048),
-                     idesc_dq, kk ? 1u : 0u);
+            umma_f16(tmem_base + COL_ST, desc_at(kt_desc, UNIT_BYTES + kk * 2048), desc_at(dsm, kk * 2048), idesc_dq,
+                     kk ? 1u : 0u);
           umma_commit(dq_hi_full);
         }
         // head elements 0..127 (units 0, 1 of K) go into the dQ^T buffer, free once the tile of the
@@ -468,15 +468,16 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       // ------------------------------------------------------ dQ reduction --
       // dQ^T (lane = head element, column = query row) is transposed through this warp's staging
       // tile as a dense fp32 [64 query rows x 32 head elements] tile, which one TMA reduce adds to
-      // the fp32 dQ in global memory.  The upper product leaves the head elements 128..191 in lanes 64..127
-      // in even steps and in lanes 0..63 in odd ones: two warps at a time pass a second tile through their
+      // the fp32 dQ in global memory.  Warps 2 and 3 own lanes 64..127, where the upper product
+      // leaves the head elements 128..191: they pass a second tile per step through the same
       // staging memory.
+      const bool has_hi = quarter >= 2;
       uint8_t* tile = sStage + quarter * STAGE_TILE;
       float* stage = reinterpret_cast<float*>(tile) + lane;
       for (int it = 0; it < n_it && ok; ++it) {
         const int q0 = (i_start + it) * BQ;
         uint32_t r[64];
-        if ((quarter >= 2) == ((it & 1) == 0)) {
+        if (has_hi) {
           // the upper tile first: the next score tile waits for its buffer
           ok = mbar_wait_bounded(dq_hi_full, it & 1, abort_flag, p.status, kTimeoutTmemFull, blockIdx.x);
           if (!ok) break;
@@ -496,7 +497,7 @@ mla_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
           fence_proxy_async();
           __syncwarp();
           if (lane == 0) {
-            tma_reduce_add_3d(&tmap_dq, tile, head * DQK + 128 + (quarter & 1) * 32, q0, batch);
+            tma_reduce_add_3d(&tmap_dq, tile, head * DQK + 128 + (quarter - 2) * 32, q0, batch);
             tma_store_commit();
           }
         }
