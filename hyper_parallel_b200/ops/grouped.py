@@ -156,8 +156,7 @@ def _expert_wgrad(a, b, out, table):
 
 
 class _Plan:
-    """Rows of a call: which padded row every (token, slot) pair takes.  One read-back of the per-expert
-    counts, which sizes the layout and refuses expert ids out of range.
+    """Rows of a call: which padded row every (token, slot) pair takes.
 
     ``table``  [E] group starts, [E] group ends, [E] counts, 1 word: an id was out of range
     ``slots``  [rows / pad] expert of each row block, [rows] pair of each row (-1: padding), [pairs] row of
@@ -168,24 +167,33 @@ class _Plan:
     def __init__(self, idx, num_experts):
         lib = _local_lib()
         dev = idx.device
-        stream = native.stream(dev)
         T, k = idx.shape
         E, pairs = num_experts, T * k
         pad = 256 if pairs >= _PAIR_MIN_ROWS * E else _BLOCK_M
-        hist = torch.empty((pairs + 255) // 256 * E, dtype=torch.int32, device=dev)
+        self.idx, self.dims = idx, (T, k, E, None, pad)
+        self.hist = torch.empty((pairs + 255) // 256 * E, dtype=torch.int32, device=dev)
         self.table = torch.empty(3 * E + 1, dtype=torch.int32, device=dev)
         starts = self.table.data_ptr()
-        native.check(lib.hpb_moe_count(idx.data_ptr(), hist.data_ptr(), starts + 8 * E, starts, starts + 4 * E, pairs, E,
-                                       pad, stream), "hpb_moe_count")
+        native.check(lib.hpb_moe_count(idx.data_ptr(), self.hist.data_ptr(), starts + 8 * E, starts, starts + 4 * E,
+                                       pairs, E, pad, native.stream(dev)), "hpb_moe_count")
+
+    def place(self):
+        """Read the per-expert counts back, which sizes the layout and refuses expert ids out of range, and
+        fill ``slots``.  (The host work between the read-back and the first product is not hidden by anything.)"""
+        T, k, E, _, pad = self.dims
+        dev = self.idx.device
         *per_expert, bad = self.table[2 * E:].tolist()
         if bad:
             raise ValueError(f"expert ids must lie in [0, {E})")
         rows = sum((c + pad - 1) // pad * pad for c in per_expert)
         self.dims = (T, k, E, rows, pad)
-        self.slots = torch.empty(rows // pad + rows + pairs, dtype=torch.int32, device=dev)
-        native.check(lib.hpb_moe_place(idx.data_ptr(), hist.data_ptr(), starts, starts + 4 * E, self.slots.data_ptr(),
-                                       _row_pair(self.slots, self.dims), _pos(self.slots, self.dims), pairs, E, pad,
-                                       rows, native.status_word(dev).data_ptr(), stream), "hpb_moe_place")
+        self.slots = torch.empty(rows // pad + rows + T * k, dtype=torch.int32, device=dev)
+        starts = self.table.data_ptr()
+        native.check(_local_lib().hpb_moe_place(
+            self.idx.data_ptr(), self.hist.data_ptr(), starts, starts + 4 * E, self.slots.data_ptr(),
+            _row_pair(self.slots, self.dims), _pos(self.slots, self.dims), T * k, E, pad, rows,
+            native.status_word(dev).data_ptr(), native.stream(dev)), "hpb_moe_place")
+        self.idx = self.hist = None
 
 
 def _row_pair(slots, dims):
@@ -210,8 +218,9 @@ class _ExpertRows(torch.autograd.Function):
         lib = _local_lib()
         dev = x.device
         stream = native.stream(dev)
-        T, k, E, rows, pad = plan.dims
         _, F2, H = w_gate_up.shape
+        plan.place()
+        T, k, E, rows, pad = plan.dims
         xp = torch.empty((rows, H), dtype=x.dtype, device=dev)
         native.check(lib.hpb_moe_gather(x.data_ptr(), _row_pair(plan.slots, plan.dims), xp.data_ptr(), rows, k, H,
                                         T * k, native.status_word(dev).data_ptr(), stream), "hpb_moe_gather")
