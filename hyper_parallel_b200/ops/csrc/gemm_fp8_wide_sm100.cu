@@ -323,7 +323,12 @@ extern "C" int hpb_gemm_fp8_blockscale_wide(const void* Aq, const float* sa, con
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || !configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_fp8_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    // the promotion warps' registers come out of what the CTA launches with: less would leave them waiting for good
+    cudaFuncAttributes fa;
+    cudaError_t e = cudaFuncGetAttributes(&fa, gemm_fp8_wide_kernel);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    if (fa.numRegs * THREADS < 128 * PRODUCER_REGS + PROMO_WARPS * 32 * PROMO_REGS) return -6;
+    e = cudaFuncSetAttribute(gemm_fp8_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     if (e != cudaSuccess) return static_cast<int>(e);
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }

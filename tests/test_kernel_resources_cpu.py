@@ -21,6 +21,14 @@ def test_gemm_accumulators_stay_in_registers():
     assert not [name for name, frame in gemms if frame]
 
 
+def test_register_split_of_the_wide_fp8_kernel_fits_its_launch():
+    """``setmaxnreg.inc`` draws on the registers the CTA launched with: 640 threads, split 128 x 56 + 512 x 104."""
+    _entries()
+    log = (build.BUILD_DIR / "ptxas.log").read_text()
+    (regs,) = re.findall(r"gemm_fp8_wide_kernel[^\n]*'\s+for[^\n]*\n(?:.*\n){1,3}?.*Used (\d+) registers", log)
+    assert int(regs) * 640 >= 128 * 56 + 512 * 104
+
+
 @pytest.mark.parametrize("name", ["hpb_mla_attn_set_probe", "hpb_mla_attn_set_prof"])
 def test_no_switch_that_skips_work(name):
     """A library call must not be able to leave parts of a kernel out."""
