@@ -6,12 +6,13 @@
 // run.  Rows between a group's end and the next start are written as zeros by the gathers.
 //
 //   plan    hist     per chunk of 256 pairs: pairs per expert
-//           scan     one CTA: per expert, prefix sums over the chunks and the group starts; block table
+//           scan     one CTA: per expert, prefix sums over the chunks and the group starts
+//           tables   expert of each row block; padding rows named as such
 //           place    pair -> row: start + chunk prefix + rank inside the chunk; row -> pair
 //   gather  x[T, H] -> xp[rows, H]
-//   scatter-back kernels read the k rows of a token and sum them in fp32 (one pass, no atomics)
+//   combine / combine_bwd  the weighted fp32 sum of a token's k rows (one pass, no atomics); its gradient
 //
-// All of them stream 16-byte vectors and are bound by HBM.  The index_copy / index_select / index_add
+// The last three stream 16-byte vectors and are bound by HBM.  The index_copy / index_select / index_add
 // sequence they take the place of moved each row through memory eight times and added bf16 values
 // atomically: 8.0 of 17.4 ms for 4096 tokens x 8 of 32 experts, hidden 7168, forward + backward.  With
 // these kernels (0.5 ms) and the expert products on CTA pairs the layer takes 8.4-9.6 ms, and 1.90 instead

@@ -176,7 +176,8 @@ class _RopeTail(torch.autograd.Function):
 def rope_tail_(x: torch.Tensor, dr: int, seq_len: int, theta: float) -> torch.Tensor:
     """Rotate the last ``dr`` columns of every head of ``x[T, NH, D]`` (positions ``t % seq_len``) in
     place and return ``x``; differentiable (the input must not be needed by the op that produced it,
-    which holds for a projection output)."""
+    which holds for a projection output).  For a per-head view at hand; the models rotate the packed
+    projection itself (``rope_tail_packed_``)."""
     return _RopeTail.apply(x, dr, seq_len, theta)
 
 
