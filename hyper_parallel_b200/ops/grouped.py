@@ -276,14 +276,17 @@ def _combine_rows(yp, gate, slots, dims):
 
 
 class _Combine(torch.autograd.Function):
-    """``y[t] = sum_j gate[t, j] * yp[row of (t, j)]``; ``gate`` fp32, contiguous.  A node of its own, so
-    that the gate weights keep their higher derivatives (the products of the experts have none)."""
+    """``y[t] = sum_j gate[t, j] * yp[row of (t, j)]``.  A node of its own, so that the gate weights keep their
+    higher derivatives (the products of the experts have none).  The backward pass multiplies with a private
+    copy of the gate, which a caller may overwrite; ``gate`` itself stands for its history only."""
 
     @staticmethod
     def forward(ctx, yp, gate, plan):
-        ctx.save_for_backward(yp if ctx.needs_input_grad[1] else None, gate, plan.slots)
+        own = gate.to(torch.float32, copy=True, memory_format=torch.contiguous_format)
+        ctx.save_for_backward(yp if ctx.needs_input_grad[1] else None, own, plan.slots)
+        ctx.gate, ctx.version = gate, gate._version
         ctx.dims, ctx.like = plan.dims, (yp.dtype, yp.shape[1])
-        return _combine_rows(yp, gate, plan.slots, plan.dims)
+        return _combine_rows(yp, own, plan.slots, plan.dims)
 
     @staticmethod
     def backward(ctx, dy):
@@ -294,12 +297,18 @@ class _Combine(torch.autograd.Function):
         dyp = dgate = None
         if torch.is_grad_enabled() or not torch._C._has_storage(dy):
             # a graph of the gradients, or a batch of them, is wanted: the same sums as tensor operations
+            if torch.is_grad_enabled():
+                if ctx.gate._version != ctx.version:
+                    raise RuntimeError("the gate weights were overwritten after the forward pass; a graph of their "
+                                       "gradients needs them")
+                gate = ctx.gate.float()
             pos = _pos_tensor(slots, ctx.dims)
             if need_rows:
                 dyp = torch.zeros((rows, H), dtype=dtype, device=dy.device).index_copy(
                     0, pos.view(-1), (gate[:, :, None] * dy[:, None].float()).to(dtype).reshape(T * k, H))
             if need_gate:
-                dgate = torch.stack([(dy.float() * yp.index_select(0, pos[:, j]).float()).sum(-1) for j in range(k)], -1)
+                dgate = torch.stack([(dy.float() * yp.index_select(0, pos[:, j]).float()).sum(-1) for j in range(k)],
+                                    -1).to(ctx.gate.dtype)
             return dyp, dgate, None
         dy = _rows16(dy)
         dyp = torch.empty((rows, H), dtype=dtype, device=dy.device)
@@ -308,7 +317,7 @@ class _Combine(torch.autograd.Function):
                                                       native.ptr(yp), dyp.data_ptr(), native.ptr(dgate), rows, k, H,
                                                       T * k, native.status_word(dy.device).data_ptr(),
                                                       native.stream(dy.device)), "hpb_moe_combine_bwd")
-        return dyp, dgate, None
+        return dyp, dgate.to(ctx.gate.dtype) if need_gate else None, None
 
 
 def _plain(t: torch.Tensor) -> bool:
@@ -332,14 +341,12 @@ def local_experts(x, topk_idx, topk_w, w_gate_up, w_down):
     (``moe_local.cu`` around the grouped GEMMs)."""
     plan = _Plan(topk_idx.contiguous(), w_gate_up.shape[0])
     yp = _ExpertRows.apply(_rows16(x), _rows16(w_gate_up), _rows16(w_down), plan)
-    # a copy: a caller may overwrite its gate weights before the backward pass
-    gate = topk_w.to(torch.float32, copy=True, memory_format=torch.contiguous_format)
-    if torch.autograd.forward_ad.unpack_dual(gate).tangent is not None:
-        pos = _pos_tensor(plan.slots, plan.dims)
+    if torch.autograd.forward_ad.unpack_dual(topk_w).tangent is not None:
+        pos, gate = _pos_tensor(plan.slots, plan.dims), topk_w.float()
         return sum(gate[:, j, None] * yp.index_select(0, pos[:, j]).float() for j in range(pos.shape[1])).to(x.dtype)
-    if not (torch.is_grad_enabled() and (yp.requires_grad or gate.requires_grad)):
-        return _combine_rows(yp, gate, plan.slots, plan.dims)
-    return _Combine.apply(yp, gate, plan)
+    if torch.is_grad_enabled() and (yp.requires_grad or topk_w.requires_grad):
+        return _Combine.apply(yp, topk_w, plan)
+    return _combine_rows(yp, topk_w.to(torch.float32).contiguous(), plan.slots, plan.dims)
 
 
 def _rows16(t: torch.Tensor) -> torch.Tensor:
